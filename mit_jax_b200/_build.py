@@ -6,8 +6,8 @@ import sys
 from pathlib import Path
 
 HERE = Path(__file__).resolve().parent
-SOURCES = [HERE / "csrc" / "cg2d_solver.cu", HERE / "csrc" / "cg2d_capi.cu", HERE / "csrc" / "cg2d_adjoint.cu",
-           HERE / "csrc" / "cg2d_pressure.cu"]
+SOURCES = [HERE / "csrc" / "cg2d_solver.cu", HERE / "csrc" / "cg2d_team.cu", HERE / "csrc" / "cg2d_capi.cu",
+           HERE / "csrc" / "cg2d_adjoint.cu", HERE / "csrc" / "cg2d_pressure.cu"]
 OUT = HERE / "libcg2d.so"
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
               "-Xcompiler", "-fPIC"]
@@ -52,7 +52,7 @@ def build_ffi(force=False):
 
 def build(force=False, verbose=False):
     """Compile the translation units side by side into objects next to the library, then link libcg2d.so."""
-    deps = SOURCES + [HERE / "csrc" / "cg2d_internal.cuh", HERE.parent / "include" / "cg2d.h"]
+    deps = SOURCES + [HERE / "csrc" / "cg2d_internal.cuh", HERE / "csrc" / "cg2d_device.cuh", HERE.parent / "include" / "cg2d.h"]
     if not force and OUT.exists() and all(OUT.stat().st_mtime >= d.stat().st_mtime for d in deps):
         return OUT
     objs = [HERE / "csrc" / (src.stem + ".o") for src in SOURCES]

@@ -56,7 +56,21 @@ struct WsLayout {
   int ch, nw, rpb, nstage[P_NPASS];   // chunk rows, compute warps, ROWBLOCK block rows
   unsigned stage_bytes;
   size_t smem;
+  // solves with their state on chip (cg2d_team.cu), when every group fits: the zeroed area runs to t_zero_end
+  bool team;
+  TeamDev t[kMaxGroups];
+  size_t t_smem[kMaxGroups], t_zero_end, t_hist, t_coef[kMaxGroups], t_msg[kMaxGroups], t_x[kMaxGroups];
 };
+
+int sm_count() {
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    cudaGetLastError();
+    return 148;
+  }
+  return n;
+}
 
 inline int round_up(int x, int m) { return (x + m - 1) / m * m; }
 
@@ -126,6 +140,47 @@ cg2d_status_t size_stages(const cg2d_group_t* gr, int ng, int mixed, int serial,
     }
   }
   return CG2D_UNSUPPORTED;
+}
+
+// The launch in teams: taken whenever every group has the same number of right-hand sides and one instance's state fits
+// in the shared memory of the CTAs the launch may use (one per SM, at most grid_ctas). One LLC90 FP64 solve: 6.4 ms
+// streamed (cg2d_solver.cu), see cg2d_team.cu for the times in teams. What is larger streams.
+void team_layout(const cg2d_group_t* gr, int ng, const cg2d_params_t* p, WsLayout* L) {
+  const bool mixed = p->precision == CG2D_PREC_MIXED, serial = p->sum_order == CG2D_SUM_FORTRAN;
+  int ctas = sm_count();
+  if (p->grid_ctas > 0 && p->grid_ctas < ctas) ctas = p->grid_ctas;
+  L->team = false;
+  for (int g = 0; g < ng; ++g) {
+    if (gr[g].nrhs != gr[0].nrhs) return;
+    TeamDev& t = L->t[g];
+    std::memset(&t, 0, sizeof(t));
+    t.nblk = L->nblk[g];
+    t.units = L->units[g];
+    t.rpb = serial ? gr[g].topo->sNy : L->rpb;
+    L->t_smem[g] = team_plan(topo_dev(gr[g].topo), gr[g].count, gr[g].nrhs, mixed, serial, ctas, &t);
+    if (L->t_smem[g] == 0) return;
+  }
+  L->team = true;
+  size_t o = L->zero_end;
+  for (int g = 0; g < ng; ++g) {
+    TeamDev& t = L->t[g];
+    t.msg_stride = (long long)al(team_msg_bytes(topo_dev(gr[g].topo), gr[g].nrhs, mixed, t));
+    L->t_msg[g] = o;
+    o += (size_t)t.msg_stride * t.nteams;
+  }
+  L->t_zero_end = o;
+  L->t_hist = o;
+  o += al(sizeof(double) * (size_t)L->total_rhs * H_NKIND * L->hist_len);
+  for (int g = 0; g < ng; ++g) {
+    TeamDev& t = L->t[g];
+    const cg2d_topology* tp = gr[g].topo;
+    t.x_stride = (long long)tp->nTiles * tp->sNy * tp->sNx * gr[g].nrhs;
+    L->t_x[g] = o;
+    o += al(sizeof(double) * (size_t)t.x_stride * t.nteams);
+    L->t_coef[g] = o;
+    o += al(team_coef_bytes(topo_dev(tp), mixed, t) * t.nteams);
+  }
+  if (o > L->total) L->total = o;
 }
 
 cg2d_status_t compute_layout(const cg2d_group_t* gr, int ng, const cg2d_params_t* p, WsLayout* L) {
@@ -202,6 +257,7 @@ cg2d_status_t compute_layout(const cg2d_group_t* gr, int ng, const cg2d_params_t
     o += al(vsz * 2 * (size_t)tp->nTiles * (tp->sNy + 1) * 3 * coef_pitch(tp->sNx) * gr[g].count);
   }
   L->total = o;
+  team_layout(gr, ng, p, L);
   return CG2D_OK;
 }
 
@@ -365,6 +421,35 @@ struct CkRec {
   int* hist_len;
 };
 
+// the launch of kp's groups in teams (cg2d_team.cu)
+static cg2d_status_t launch_in_teams(const KParams& kp, const WsLayout& L, char* ws, cudaStream_t stream) {
+  cudaError_t e = cudaMemsetAsync(ws, 0, L.t_zero_end, stream);
+  for (int g = 0; g < kp.ngroups && e == cudaSuccess; ++g) {   // one launch per group
+    TeamParams tp;
+    std::memset(&tp, 0, sizeof(tp));
+    tp.g = kp.g[g];
+    tp.t = L.t[g];
+    tp.t.msg = ws + L.t_msg[g];
+    tp.t.x = reinterpret_cast<double*>(ws + L.t_x[g]);
+    tp.replace_every = kp.replace_every;
+    tp.replace_above = kp.replace_above;
+    tp.hist = kp.hist;
+    tp.hist_len = kp.hist_len;
+    tp.gs = kp.gs;
+    tp.timeout_ns = kp.timeout_ns;
+    tp.test_missing = kp.test_missing;
+    tp.prof = kp.prof;
+    tp.ck_r = kp.ck_r;
+    tp.ck_s = kp.ck_s;
+    tp.ck_stride = kp.ck_stride;
+    tp.ck_every = kp.ck_every;
+    tp.t.coef = ws + L.t_coef[g];
+    e = launch_team(tp, kp.mixed, kp.serial, L.t_smem[g], stream);
+  }
+  if (e != cudaSuccess) { cudaGetLastError(); return CG2D_CUDA_ERROR; }
+  return CG2D_OK;
+}
+
 static cg2d_status_t solve_groups_impl(const cg2d_group_t* groups, int ngroups, const cg2d_params_t* params,
                                        void* workspace, size_t workspace_bytes, cg2d_stream_t stream_,
                                        const CkRec* ck) {
@@ -403,7 +488,7 @@ static cg2d_status_t solve_groups_impl(const cg2d_group_t* groups, int ngroups, 
   kp.ch = L.ch;
   for (int i = 0; i < P_NPASS; ++i) kp.nstage[i] = L.nstage[i];
   kp.stage_bytes = L.stage_bytes;
-  kp.hist = reinterpret_cast<double*>(ws + L.hist);
+  kp.hist = reinterpret_cast<double*>(ws + (L.team ? L.t_hist : L.hist));
   kp.hist_len = L.hist_len;
   kp.part = reinterpret_cast<double*>(ws + L.part);
   kp.part_units = L.part_units;
@@ -468,9 +553,7 @@ static cg2d_status_t solve_groups_impl(const cg2d_group_t* groups, int ngroups, 
   }
 
   const size_t smem = L.smem;
-  int dev = 0, nsm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  const int nsm = sm_count();
   // FP64 has a kernel built for 1 CTA per SM (no register limit below the SM's) and one for 2 (96 registers a
   // thread). ctas_per_sm 2 takes the second; 0 takes it when every group has one right-hand side and there are at
   // least 8 units per SM, where its doubled warps pay for the spills (exact-mode forward solves); otherwise the first.
@@ -490,6 +573,7 @@ static cg2d_status_t solve_groups_impl(const cg2d_group_t* groups, int ngroups, 
   if (grid > kMaxCtas) grid = kMaxCtas;
   if (grid < 1) grid = 1;
   if ((kp.total_units + grid - 1) / grid > kMaxUnitsPerCta) return CG2D_UNSUPPORTED;   // unit table of a CTA
+  if (L.team) return launch_in_teams(kp, L, ws, stream);
   if (cudaMemsetAsync(ws, 0, L.zero_end, stream) != cudaSuccess) { cudaGetLastError(); return CG2D_CUDA_ERROR; }
   for (int g = 0; g < ngroups; ++g)
     if (launch_pack_coef(kp.g[g], kp.mixed, stream) != cudaSuccess) { cudaGetLastError(); return CG2D_CUDA_ERROR; }

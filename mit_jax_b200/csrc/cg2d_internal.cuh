@@ -191,6 +191,48 @@ constexpr int kMaxCtas = 148 * 8;
 enum ProfPhase : int { PR_BAR = 0, PR_MBAR = 1, PR_ISSUE = 2, PR_COMP = 3, PR_FIN = 4, PR_DIRECT = 5, PR_OTHER = 6,
                        PR_TOTAL = 7, PR_DRAIN = 8, PR_RWAIT = 9, PR_CTRL = 10, PR_PWAIT = 11, kProfSlots = 12 };
 
+// ---- teams: solves whose state stays in shared memory (cg2d_team.cu)
+constexpr int kTeamWarps = 16;             // warps per CTA (one CTA per SM)
+constexpr int kTeamThreads = kTeamWarps * 32;
+constexpr int kTeamMaxCtas = 160;          // CTAs of a team
+constexpr int kTeamKinds = 3;              // sums of one exchange: r.r, z.r and, at the start, the sum of b
+
+// How one group of a launch runs in teams. A team is G consecutive CTAs; it solves one instance after another (instance
+// team, team + nteams, ...). The instance's work units (tile, row block) are dealt to its CTAs in contiguous runs:
+// CTA c of a team owns units ub[c] .. ub[c + 1] - 1.
+struct TeamDev {
+  int G, nteams;
+  int nblk, units, rpb;           // work units per tile / per instance, rows per unit
+  int max_rows, max_units;        // rows and units of the largest CTA
+  int sum_block;                  // sum messages of a CTA: [sums][max_units], in 128-byte lines of its own
+  long long nslots;               // halo messages of an instance: west / east points by row, then first / last unit rows
+  char* msg;                      // per team: 2 x [message kinds][nslots] halo messages, then 2 x [G][sum_block] sums
+  long long msg_stride;           // bytes
+  void* coef;                     // per CTA: packed coefficients [2][max_rows][ni + 1] x (west, south, north, centre)
+  double* x;                      // per team: the solution [T nj ni][nrhs]
+  long long x_stride;             // elements
+  // shared memory of a CTA (bytes from the start of its dynamic area)
+  unsigned o_rows, o_units, o_halo, o_send, o_umsg, o_hval, o_rowsum, o_psum, o_tsum, o_r, o_s, o_q;
+  unsigned ring_elems;            // elements of r and of s
+  unsigned short ub[kTeamMaxCtas + 1];
+};
+struct TeamParams {   // one group
+  GroupDev g;
+  TeamDev t;
+  int replace_every;
+  double replace_above;
+  double* hist;                   // as KParams
+  int hist_len;
+  unsigned* gs;
+  unsigned long long timeout_ns;
+  int test_missing;               // testing: the first exchange of a team waits for a message that nobody sends
+  unsigned long long* prof;
+  double* ck_r;
+  double* ck_s;
+  long long ck_stride;
+  int ck_every;
+};
+
 // exact-mode adjoint (cg2d_adjoint.cu)
 struct ExactArgs {
   int batch, max_iters, checkpoint, rows_per_block;
@@ -217,6 +259,13 @@ cudaError_t exact_adjoint(const TopoDev& tp, const ExactArgs& args, void* worksp
 size_t fixed_smem_bytes(int max_ni, int serial);
 cudaError_t launch_solver(const KParams& kp, int grid, size_t smem, cudaStream_t stream);
 cudaError_t solver_occupancy(const KParams& kp, size_t smem, int* blocks_per_sm);
+
+// One group's team plan on `ctas` CTAs (one per SM): fills G, nteams, ub and the shared-memory layout of t (its nblk, units, rpb
+// and the group's tp, count, nrhs are set) and returns a CTA's dynamic shared memory, or 0 when no split fits.
+size_t team_plan(const TopoDev& tp, int count, int nrhs, int mixed, int serial, int ctas, TeamDev* t);
+size_t team_msg_bytes(const TopoDev& tp, int nrhs, int mixed, const TeamDev& t);   // per team
+size_t team_coef_bytes(const TopoDev& tp, int mixed, const TeamDev& t);            // per team
+cudaError_t launch_team(const TeamParams& kp, int mixed, int serial, size_t smem, cudaStream_t stream);
 cudaError_t launch_pack_coef(const GroupDev& g, int mixed, cudaStream_t stream);
 cudaError_t launch_apply_operator(const TopoDev& tp, int batch, double norm, const double* aW, const double* aS,
                                   const double* aC, const double* v, double* out, cudaStream_t stream);

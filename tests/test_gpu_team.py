@@ -1,0 +1,61 @@
+"""Solves whose state stays on chip (csrc/cg2d_team.cu) where the split of the work can go wrong: tiles of one or a few
+rows per work unit, runs of rows over tile edges, one CTA per team and many, more instances than teams, rows of one and
+several column steps, both right-hand sides, both precisions, both sum orders. grid_ctas limits the CTAs, so the same solve
+runs in other team sizes and, where its state does not fit them, streamed (csrc/cg2d_solver.cu). Every variant performs the
+same additions in the same order: solutions, halos and diagnostics are equal bit for bit."""
+
+import pytest
+import torch
+
+from mit_jax_b200 import cg2d as cg
+from mit_jax_b200.synthetic import make_batch
+from oracle import cg2d_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    # N, ts, instances, right-hand sides, precision, sum order, rows per block, CTA limits
+    (8, 8, 1, 1, "f64", "rowblock", 8, (1, 5, 13)),
+    (8, 2, 1, 2, "f64", "fortran", 8, (1, 7, 148)),
+    (20, 10, 3, 1, "f64", "rowblock", 8, (1, 2, 17, 148)),
+    (34, 34, 2, 1, "f64", "rowblock", 16, (2, 9, 148)),
+    (36, 12, 5, 2, "mixed", "rowblock", 8, (3, 40, 148)),
+    (66, 66, 2, 1, "mixed", "rowblock", 8, (4, 30, 148)),
+    (90, 90, 3, 2, "mixed", "rowblock", 8, (4, 26, 148)),
+    (90, 90, 2, 1, "f64", "fortran", 8, (4, 13, 148)),
+    (98, 98, 1, 2, "f64", "rowblock", 24, (4, 100, 148)),
+    (130, 130, 1, 1, "mixed", "fortran", 8, (4, 60, 148)),
+    (194, 194, 1, 1, "f64", "rowblock", 8, (4, 90, 148)),
+]
+
+
+def _group(N, ts, count, nrhs, iters):
+    syn, B = make_batch(N, count, ts, with_cotangent=True, members=list(range(count)))
+    ex = cg.Exchanger(syn.L, syn.topo.maps)
+    t = {k: torch.as_tensor(v).cuda() for k, v in B.items()}
+    x0 = 0.01 * t["w"]
+    return syn, B, cg.GroupSpec(ex, tuple(t[k] for k in cg.OPS), [t["b"], t["w"]][:nrhs], [x0, 0.5 * x0][:nrhs],
+                                [1e-9, 1e-6][:nrhs], [iters, iters][:nrhs], t["cg2dNorm"], x_fortran=True)
+
+
+@pytest.mark.parametrize("N,ts,count,nrhs,precision,order,rows,limits", CASES)
+def test_every_split_is_bitwise_equal(N, ts, count, nrhs, precision, order, rows, limits):
+    _, _, G = _group(N, ts, count, nrhs, 70)
+    kw = dict(precision=precision, sum_order=order, rows_per_block=rows)
+    (ref,) = cg.solve_groups([G], **kw)
+    for limit in limits:
+        (got,) = cg.solve_groups([G], grid_ctas=limit, **kw)
+        for (x0, f0, d0), (x1, f1, d1) in zip(ref, got):
+            assert torch.equal(x0, x1) and torch.equal(f0, f1) and torch.equal(d0, d1), limit
+
+
+def test_more_instances_than_teams_equal_the_oracle():
+    syn, B, G = _group(24, 12, 23, 1, 60)
+    ((x, xf, dg),) = cg.solve_groups([G], sum_order="rowblock", grid_ctas=20)[0]
+    recs = cg.diag_records(dg)
+    for m in (0, 11, 22):
+        ops = tuple(B[k][m] for k in cg.OPS)
+        xo, do = O.cg2d_fortran(syn.L, syn.topo.maps["T"], ops, B["b"][m], 0.01 * B["w"][m],
+                                cg2dNorm=B["cg2dNorm"][m], tolerance=1e-9, max_iters=60, sum_order="rowblock")
+        assert recs[m]["numIters"] == do["numIters"]
+        assert torch.equal(xf[m].cpu(), torch.as_tensor(xo))
