@@ -435,7 +435,8 @@ struct Team {
     }
   }
 
-  // the total of each of the n sums from psum, in fixed order, into sc().total
+  // the total of each of the n sums from psum, in fixed order: tile sums by all threads, then (warp 0) the totals into
+  // sc().total
   __device__ __forceinline__ void fold(int n) {
     const int nb = kp.t.nblk, nt = kp.g.tp.T;
     for (int e = threadIdx.x; e < n * nt; e += kTeamThreads) {
@@ -452,21 +453,22 @@ struct Team {
       tsum()[e] = a;
     }
     __syncthreads();
-    // sum q by warp q: its lanes hold 32 tile sums, every lane adds them in order
-    const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (q < n) {
-      const double* p = tsum() + q * nt;
-      double a = 0.0;
-#pragma unroll 1
-      for (int t = 0; t < nt; t += 32) {
-        const double v = t + lane < nt ? p[t + lane] : 0.0;
-        const int m = min(32, nt - t);
-#pragma unroll 8
-        for (int k = 0; k < m; ++k) a = add(a, __shfl_sync(0xffffffffu, v, k));
+    if (threadIdx.x < 32) {
+      if ((int)threadIdx.x < n) {
+        const double* p = tsum() + threadIdx.x * nt;
+        double a = 0.0;
+        for (int t = 0; t < nt; t += 13) {
+          double v[13];
+#pragma unroll
+          for (int c = 0; c < 13; ++c) v[c] = t + c < nt ? p[t + c] : 0.0;
+#pragma unroll
+          for (int c = 0; c < 13; ++c)
+            if (t + c < nt) a = add(a, v[c]);
+        }
+        sc().total[threadIdx.x] = a;
       }
-      if (lane == 0) sc().total[q] = a;
+      __syncwarp();
     }
-    __syncthreads();
   }
 
   __device__ __forceinline__ long long pad_of(int grow, int i) const {
@@ -664,9 +666,8 @@ struct Team {
         }
 #pragma unroll 1
         for (; lr < end; ++lr) {
-          Coefs f1;
-          f1.w = (C)0;
-          load(f1, cf, min(lr + 1, lrB - 1), 0);
+          Coefs f1 = f;
+          if (lr + 1 < lrB) load(f1, cf, lr + 1, 0);
 #pragma unroll
           for (int m = 0; m < STEPS; ++m) {
             const int x = m < L ? 32 * m : last;
