@@ -375,9 +375,8 @@ def run_gpu(a):
         prof = cg.solve_groups.last_profile.astype(np.float64) / 1e6
         phases = {"per_cta_mean": {n: float(prof[:, i].mean()) for i, n in enumerate(cg.PROF_NAMES)},
                   "ctas": int(prof.shape[0]),
-                  "note": "ms per CTA over one launch: bar grid-wide waits, mbar waits for stage data, comp chunk "
-                          "compute, fin/direct/drain/other the rest of thread 0's time; issue and pwait the copy "
-                          "warp's busy and waiting time"}
+                  "note": "ms of thread 0 per CTA over one launch: bar waits for messages, comp the stencils, ctrl the vector "
+                          "updates, direct the x update, issue forming and sending sums, fin the totals and scalars"}
 
     # ---- end to end through the public API from pinned host buffers. Every step uploads its inputs and
     #      downloads its solutions, gradients and diagnostics; the steps are pipelined over three streams (step s+1's
@@ -494,7 +493,7 @@ def run_gpu(a):
             "config": arm_config(a, world),
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind,
-                         "kernel": "cg2d_persistent (solver launch incl. FP32 pack)",
+                         "kernel": "cg2d_team (the solver launch)",
                          "kernel_ms": solver_mean, "algorithmic_bytes_per_launch": alg,
                          "coefficients_counted_once": {
                              "algorithmic_bytes_per_launch": alg - shared,
@@ -503,7 +502,7 @@ def run_gpu(a):
                                      "solves; the paired launch reads them once"}},
             "cpu_baseline": cpu,
             "e2e": e2e,
-            "gpu_launches": 3 * a.steps,
+            "gpu_launches": 2 * a.steps,   # the solve (one team launch) and the edge products
             "clocks": clocks,
             "iterations": {"fwd_mean": statistics.mean(d["numIters"] for d in diag_f),
                            "adj_mean": statistics.mean(d["numIters"] for d in diag_a),
@@ -554,13 +553,13 @@ def exact_algorithmic_bytes(iters, checkpoint):
 
 def exact_launches(kmax, checkpoint):
     """Kernels one cg2d_solve_exact call launches for a batch whose largest iteration count is kmax (memsets
-    excluded): the coefficient pack and the solve; set-up, neighbour table, r_0 and the scalars from the solve's
+    excluded): the solve; set-up, neighbour table, r_0 and the scalars from the solve's
     sums; the cotangent scaling; per iteration two recompute kernels (k_fa, k_fb) and four reverse kernels
     (k_rev_alpha, k_rq, k_rev_beta, k_rz); per segment the alphabar row dots and the two edge-product launches; and
     the two closing kernels."""
     C = checkpoint if checkpoint > 0 else max(1, kmax)
     nseg = -(-kmax // C) if kmax else 0
-    return 2 + 4 + 1 + 6 * kmax + 3 * nseg + 2
+    return 1 + 4 + 1 + 6 * kmax + 3 * nseg + 2
 
 
 def _cpu_exact(B, syn, member, iters):
@@ -843,7 +842,7 @@ def run_pressure(a):
         "steps_gbs": {"update_cg2d": gbs(upd_b, upd_ms), "cg2d_rhs": gbs(rhs_b, rhs_ms),
                       "cg2d_solve": gbs(solve_alg, solve_ms), "post": gbs(post_b, post_ms)},
         "cpu_baseline": cpu, "e2e": None,
-        "gpu_launches": a.steps * 6,
+        "gpu_launches": a.steps * 5,
         "clocks": clocks,
         "iterations": {"mean": statistics.mean(r["numIters"] for r in recs), "not_ok":
                        sum(r["status"] != "ok" for r in recs)},
@@ -925,10 +924,10 @@ def run_mixed_sizes(a):
                    "grid": "LLC270 13x270x270 and LLC90 13x90x90, halo 4", "l2": "inputs larger than L2 (no flush)",
                    "parallelism": "1 GPU"},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                     "traffic": None, "peak_kind": peak_kind, "kernel": "cg2d_persistent (mixed, two groups)",
+                     "traffic": None, "peak_kind": peak_kind, "kernel": "cg2d_team (mixed, one launch per group)",
                      "kernel_ms": ms, "algorithmic_bytes_per_launch": alg},
         "error_vs_f64": errs, "iterations": iters, "not_ok": bad,
-        "cpu_baseline": None, "e2e": None, "gpu_launches": 3 * a.steps, "clocks": clocks,
+        "cpu_baseline": None, "e2e": None, "gpu_launches": 2 * a.steps, "clocks": clocks,
         "schedule": {"chosen": sched, "launch": "CUDA graph replay"},
     }
     print(json.dumps(line))

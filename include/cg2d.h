@@ -68,7 +68,9 @@ typedef struct {
                           the 16-warp build and uses blocks of 15 rows instead */
   int replace_every;   /* MIXED: FP64 true-residual replacement period in iterations (default 25) */
   double replace_above;/* MIXED: replace only while the residual is above replace_above * tolerance (default 100) */
-  int grid_ctas;       /* 0 = as many as can be co-resident (capped by the work units) */
+  int grid_ctas;       /* 0 = as many as can be co-resident (capped by the work units). Solves whose state fits in the
+                          shared memory of these CTAs keep it there (teams of CTAs, one per SM); larger ones stream it.
+                          ctas_per_sm, unit_deal and stages concern the streaming kernel only */
   int ctas_per_sm;     /* 0 = occupancy maximum. FP64 has two kernel builds: for 1 CTA per SM and for 2 (fewer
                           registers a thread). 2 takes the second; 0 takes it when every group has one right-hand
                           side and there are at least 8 work units per SM, otherwise the first. Results-neutral */
@@ -145,7 +147,8 @@ void cg2d_default_params(cg2d_params_t* p);
 /* Bytes of device workspace a cg2d_solve_groups call with these groups needs. */
 size_t cg2d_workspace_size(const cg2d_group_t* groups, int ngroups, const cg2d_params_t* params);
 
-/* Solve every right-hand side of every group in ONE persistent cooperative launch.
+/* Solve every right-hand side of every group: one persistent cooperative launch per group when every group has the
+ * same number of right-hand sides and one instance's state fits on chip, else ONE persistent launch for all groups.
  * The workspace (device, >= cg2d_workspace_size bytes, 256-byte aligned) is scratch; it is not
  * read before being written. Returns CG2D_OK when the work was enqueued; per-solve outcomes
  * (convergence, NaN, barrier timeout) are in each solve's diag.status. */
@@ -342,6 +345,8 @@ cg2d_status_t cg2d_exchange_scalar(const cg2d_topology_t* topo, int batch, const
  *                    the copy warp's last row sums, [9] reducer waits for unit counts (within [4]),
  *                    [10] control code between passes;
  *   the copy warp:   [2] busy issuing copies and folding row sums, [11] waiting for the compute warps.
+ * Solves kept on chip: [0] waits for messages, [2] forming and sending sums, [3] stencils, [4] totals and scalars,
+ * [5] the x update, [10] vector updates, [6] the rest, [7] total; the others 0.
  * Returns CG2D_BAD_ARG when the groups/params do not describe that workspace's layout. */
 cg2d_status_t cg2d_workspace_profile(const void* workspace, const cg2d_group_t* groups, int ngroups,
                                      const cg2d_params_t* params, uint64_t* out, int cap, cg2d_stream_t stream);

@@ -143,8 +143,9 @@ cg2d_status_t size_stages(const cg2d_group_t* gr, int ng, int mixed, int serial,
 }
 
 // The launch in teams: taken whenever every group has the same number of right-hand sides and one instance's state fits
-// in the shared memory of the CTAs the launch may use (one per SM, at most grid_ctas). One LLC90 FP64 solve: 6.4 ms
-// streamed (cg2d_solver.cu), see cg2d_team.cu for the times in teams. What is larger streams.
+// in the shared memory of the CTAs the launch may use (one per SM, at most grid_ctas). Where both run, the team is faster
+// at every size measured (ms streamed, in teams): LLC32 FORTRAN order 1.8, 0.86; LLC90 FP64 x1 6.9, 2.3; 64 FP64 solves 52,
+// 29; 64 mixed pairs 48, 31; LLC270 FP64 54, 16. What does not fit streams.
 void team_layout(const cg2d_group_t* gr, int ng, const cg2d_params_t* p, WsLayout* L) {
   const bool mixed = p->precision == CG2D_PREC_MIXED, serial = p->sum_order == CG2D_SUM_FORTRAN;
   int ctas = sm_count();

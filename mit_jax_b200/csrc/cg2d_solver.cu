@@ -1,4 +1,6 @@
-// Persistent cooperative CG2D solver for sm_100a.
+// Persistent cooperative CG2D solver for sm_100a, streaming: for solves whose state does not fit in the shared memory of
+// the CTAs of a launch, and for groups with different numbers of right-hand sides in one launch. The others keep their
+// state on chip (cg2d_team.cu).
 //
 // One launch runs every right-hand side of every instance to convergence. The iteration is the
 // preconditioned CG of mitgcm_jax/core/cg2d.py:205-269 (cg2d.F), with the same floating-point

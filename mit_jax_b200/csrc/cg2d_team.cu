@@ -20,8 +20,13 @@
 // fit runs in cg2d_solver.cu, which streams the state. The arithmetic, the sum order and the results are those of
 // cg2d_solver.cu bit for bit, in every precision and sum order.
 //
-// What bounds it: per pass the message latency, the block barriers between the phases and the shared-memory and
-// coefficient reads of max_rows rows; HBM only carries inputs and outputs.
+// What bounds it. One LLC90 FP64 solve: 2.3 ms, 4.6 us a pass (6.9 ms and 14 us when streamed): the message latency (an
+// all-to-all of 148 CTAs takes 1.3 us when every CTA's sums have 128-byte lines of their own, 3.2 us when CTAs share
+// lines), the block barriers and short dependent steps between the phases. Batches: the shared-memory / L1 pipe. With 11
+// teams of 13 CTAs (mixed pairs) it is busy 54 % of the time, DRAM 2 %, issue slots 37 %; 64 mixed pairs take 31 ms (48
+// streamed), 64 FP64 solves 29 ms (52). One LLC270 FP64 solve: 16 ms (54).
+// Two CTAs of 8 warps per SM, so that one team computes while another waits, measured the same (16 FP64 solves 8.7 ms
+// either way) and fit fewer teams.
 
 #include <cuda_runtime.h>
 
@@ -1320,8 +1325,9 @@ size_t team_plan(const TopoDev& tp, int count, int nrhs, int mixed, int serial, 
   t->nslots = (2ll * rows + 2ll * t->units * ni + 7) & ~7ll;   // (whole 128-byte lines)
   if (t->nslots > (1ll << 30)) return 0;
   const unsigned es = (mixed ? 4u : 8u) * nrhs;
-  // time of a pass: the exchange, and the rows of the largest CTA at kRowCost each (units of an exchange) per 32 columns
-  // and warp
+  // time of a pass in units of an exchange (4.2 us with its fixed steps): 1 + kRowCost per row of the largest CTA's
+  // warps and 32 columns. Measured, LLC90 FP64: 4.6 us at 8 rows a CTA, 9.1 us at 66, 10.6 us at 90. The split with the
+  // least rounds x pass time is taken: 16 solves run 8 teams of 18 CTAs, 64 solves 11 teams of 13.
   const double steps = (ni + 31) / 32, kRowCost = 0.09;
   double best = 0.0;
   size_t best_smem = 0;
