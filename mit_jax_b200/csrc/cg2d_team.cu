@@ -1395,7 +1395,9 @@ size_t team_plan(const TopoDev& tp, int count, int nrhs, int mixed, int serial, 
 cudaError_t launch_team(const TeamParams& kp, int mixed, int serial, size_t smem, cudaStream_t stream) {
   const int nrhs = kp.g.nrhs, grid = kp.t.G * kp.t.nteams;
   const void* fn = team_fn(mixed, serial, nrhs, kp.g.tp.ni);
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // The limit belongs to the function, which every thread and stream of the context shares: always the largest, so that no
+  // call lowers it between another one's setting and launch.
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
   if (e != cudaSuccess) return e;
   void* args[] = {const_cast<TeamParams*>(&kp)};
   return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kTeamThreads), args, smem, stream);
