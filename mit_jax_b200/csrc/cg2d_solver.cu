@@ -1848,7 +1848,8 @@ int solver_threads(const KParams& kp) { return (kp.nw + 1) * 32; }
 
 cudaError_t solver_occupancy(const KParams& kp, size_t smem, int* blocks_per_sm) {
   const void* fn = solver_fn(kp);
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // (the largest, as launch_team: other threads launch the same build with other sizes)
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
   if (e != cudaSuccess) return e;
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, fn, solver_threads(kp), smem);
 }

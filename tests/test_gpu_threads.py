@@ -40,8 +40,12 @@ def _args(N, count, tile, **kw):
     return (arr, 1, ctypes.byref(params), base, nbytes), (ex, b, ops, x0, x, dg, ws, params)
 
 
-def test_two_threads_with_different_shared_memory():
-    calls = [_args(90, 1, None), _args(90, 16, None)]      # 36 and 171 KB a CTA of the same team build
+@pytest.mark.parametrize("case", ["on_chip", "streamed"])
+def test_two_threads_with_different_shared_memory(case):
+    if case == "on_chip":      # 36 and 171 KB a CTA of the same team build
+        calls = [_args(90, 1, None), _args(90, 16, None)]
+    else:                      # the streaming kernel at two pipeline depths (grid_ctas too small for the state)
+        calls = [_args(90, 1, None, grid_ctas=8, ctas_per_sm=1, stages=s) for s in (2, 4)]
     stream = torch.cuda.current_stream().cuda_stream
     L = capi.lib()
     for args, _ in calls:
