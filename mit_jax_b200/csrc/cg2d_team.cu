@@ -375,8 +375,9 @@ struct Team {
   }
 
   // halo messages of step htag into hval; nsum > 0: also the sums of exchange stag, [nsum][units], into psum.
-  // A thread takes messages tid, tid + threads, ...; two loads are in flight before the first is tested.
-  __device__ __forceinline__ void receive(bool with_halo, int nsum) {
+  // A thread takes messages tid, tid + threads, ...; two loads are in flight before the first is tested. acquire: what the
+  // senders had written to memory when they sent (after a fence of theirs) is visible to the CTA afterwards.
+  __device__ __forceinline__ void receive(bool with_halo, int nsum, bool acquire = false) {
     const int nh = with_halo ? nhalo * MS : 0, n = nh + nsum * kp.t.units;
     const char* hb = halo_buf();
     const char* sb = sum_buf();
@@ -408,6 +409,7 @@ struct Team {
       take(e, p, m);
       take(f, r, w);
     }
+    if (acquire) __threadfence();
     fail = __syncthreads_or(!ok) || fail;
   }
 
@@ -950,17 +952,17 @@ struct Team {
   }
 
   // the true residual b - A x of the right-hand sides in sc().rep, in FP64 (MIXED), into the shared r; x is current. Its
-  // neighbours are read from L2 after an exchange, which makes every CTA's x visible
+  // neighbours are read from L2 after an exchange that makes every CTA's x visible: the threads that send it fence after the
+  // barrier behind the CTA's stores of x, the threads that poll it fence before the barrier in front of the reads
   __device__ void true_residual() {
     Scalars& q = sc();
-    __threadfence();
     for (int lr = threadIdx.x; lr < nrows; lr += kTeamThreads)
       for (int s = 0; s < NS; ++s) rowsum()[s * kp.t.max_rows + lr] = 0.0;
     __syncthreads();
-    send_sums(1);
-    receive(false, NS);
-    if (fail) return;
     __threadfence();
+    send_sums(1);
+    receive(false, NS, true);
+    if (fail) return;
     const TopoDev& tp = kp.g.tp;
     const int n = ni(), nj = tp.nj, lane = threadIdx.x & 31, tile0 = row0 / nj;
     const int nwe = nhalo - 2 * nrows;   // halo cells before the west / east ones

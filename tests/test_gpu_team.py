@@ -59,3 +59,19 @@ def test_more_instances_than_teams_equal_the_oracle():
                                 cg2dNorm=B["cg2dNorm"][m], tolerance=1e-9, max_iters=60, sum_order="rowblock")
         assert recs[m]["numIters"] == do["numIters"]
         assert torch.equal(xf[m].cpu(), torch.as_tensor(xo))
+
+
+@pytest.mark.parametrize("nrhs", [1, 2])
+def test_true_residual_in_every_iteration(nrhs):
+    """Mixed precision with the FP64 residual b - A x formed in every iteration: each CTA reads its neighbours' x, which they
+    have just written, so every iteration depends on those stores being visible. Bitwise equal in every split and to the
+    streaming kernel (one CTA)."""
+    _, _, G = _group(48, 16, 2, nrhs, 25)
+    kw = dict(precision="mixed", replace_every=1, replace_above=0.0)
+    (ref,) = cg.solve_groups([G], grid_ctas=1, **kw)
+    assert all(r["replacements"] == r["numIters"] > 0 for _, _, d in ref for r in cg.diag_records(d))
+    for limit in (9, 40, 148):
+        for _ in range(4):
+            (got,) = cg.solve_groups([G], grid_ctas=limit, **kw)
+            for (x0, f0, d0), (x1, f1, d1) in zip(ref, got):
+                assert torch.equal(x0, x1) and torch.equal(f0, f1) and torch.equal(d0, d1), limit
