@@ -147,6 +147,16 @@ void cg2d_default_params(cg2d_params_t* p);
 /* Bytes of device workspace a cg2d_solve_groups call with these groups needs. */
 size_t cg2d_workspace_size(const cg2d_group_t* groups, int ngroups, const cg2d_params_t* params);
 
+/* How a cg2d_solve_groups call with these groups and parameters would run (sizes and parameters decide; nothing is
+ * launched). One entry per group. */
+typedef struct {
+  int on_chip;         /* 1: an instance's state stays in the shared memory of a team of CTAs; 0: it is streamed */
+  int launch;          /* the solver launch that runs the group: 0 .. launches - 1; groups may share one */
+  int teams;           /* on_chip: instances solved side by side, else 0 */
+  int ctas_per_team;   /* on_chip: CTAs of each, else 0 */
+} cg2d_group_plan_t;
+cg2d_status_t cg2d_plan(const cg2d_group_t* groups, int ngroups, const cg2d_params_t* params, cg2d_group_plan_t* plan);
+
 /* Solve every right-hand side of every group: one persistent cooperative launch per group when every group has the
  * same number of right-hand sides and one instance's state fits on chip, else ONE persistent launch for all groups.
  * The workspace (device, >= cg2d_workspace_size bytes, 256-byte aligned) is scratch; it is not

@@ -36,7 +36,7 @@ EXPORTED = ("cg2d_topology_create", "cg2d_topology_destroy", "cg2d_default_param
             "cg2d_solve_f64_noalloc", "cg2d_adjoint_exact", "cg2d_adjoint_exact_workspace_size",
             "cg2d_update_operator", "cg2d_pressure_rhs", "cg2d_pressure_post", "cg2d_solve_mixed",
             "cg2d_adjoint_ecco_workspace_size", "cg2d_adjoint_ecco", "cg2d_solve_exact_workspace_size",
-            "cg2d_solve_exact", "cg2d_ini_norm")
+            "cg2d_solve_exact", "cg2d_ini_norm", "cg2d_plan")
 
 
 class Params(ctypes.Structure):
@@ -73,6 +73,12 @@ class Group(ctypes.Structure):
                 ("cg2dNorm", ctypes.c_double), ("cg2dNorm_per_instance", _P),
                 ("b", _D2), ("x0", _D2), ("x_out", _D2), ("x_fortran", _D2), ("diag", _D2),
                 ("tolerance", ctypes.c_double * 2), ("max_iters", ctypes.c_int * 2)]
+
+
+class GroupPlan(ctypes.Structure):
+    """cg2d_group_plan_t: how a call runs a group."""
+    _fields_ = [("on_chip", ctypes.c_int), ("launch", ctypes.c_int), ("teams", ctypes.c_int),
+                ("ctas_per_team", ctypes.c_int)]
 
 
 _LIB = None
@@ -138,6 +144,8 @@ def lib():
     L.cg2d_pressure_post.restype = i
     L.cg2d_ini_norm.argtypes = [_P, i, i, d, d] + [_P] * 8 + [_P]
     L.cg2d_ini_norm.restype = i
+    L.cg2d_plan.argtypes = [ctypes.POINTER(Group), i, ctypes.POINTER(Params), ctypes.POINTER(GroupPlan)]
+    L.cg2d_plan.restype = i
     L.cg2d_status_string.argtypes = [i]
     L.cg2d_status_string.restype = ctypes.c_char_p
     _LIB = L

@@ -284,6 +284,22 @@ def solve_groups(groups, precision="f64", sum_order="rowblock", rows_per_block=8
     return result
 
 
+def solve_plan(groups, precision="f64", sum_order="rowblock", rows_per_block=8, grid_ctas=0, ctas_per_sm=0,
+               unit_deal=0, stages=0):
+    """How solve_groups with these arguments runs each group (cg2d_plan), without running it: per group a dict of on_chip
+    (state in shared memory, else streamed), launch (the launch that runs it), teams and ctas_per_team."""
+    dev = groups[0].b[0].device
+    params = _params_struct(precision, sum_order, rows_per_block, grid_ctas=grid_ctas, ctas_per_sm=ctas_per_sm,
+                            unit_deal=unit_deal, stages=stages)
+    arr, plan = (capi.Group * len(groups))(), (capi.GroupPlan * len(groups))()
+    for g, G in zip(arr, groups):
+        g.topo, g.count, g.nrhs = G.ex.handle(dev), G.b[0].shape[0], len(G.b)
+        for s in range(len(G.b)):
+            g.tolerance[s], g.max_iters[s] = float(G.tol[s]), int(G.max_iters[s])
+    capi.check(capi.lib().cg2d_plan(arr, len(groups), ctypes.byref(params), plan), "cg2d_plan")
+    return [dict(on_chip=bool(p.on_chip), launch=p.launch, teams=p.teams, ctas_per_team=p.ctas_per_team) for p in plan]
+
+
 def diag_records(dg):
     """uint8 [count, 48] device/host buffer -> list of dicts (the reference's diag keys + status)."""
     raw = dg.cpu().numpy() if isinstance(dg, torch.Tensor) else np.asarray(dg)

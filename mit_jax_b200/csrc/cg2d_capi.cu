@@ -412,6 +412,24 @@ size_t cg2d_workspace_size(const cg2d_group_t* groups, int ngroups, const cg2d_p
   return L.total;
 }
 
+cg2d_status_t cg2d_plan(const cg2d_group_t* groups, int ngroups, const cg2d_params_t* params, cg2d_group_plan_t* plan) {
+  cg2d_params_t def;
+  if (!params) { cg2d_default_params(&def); params = &def; }
+  if (!plan) return CG2D_BAD_ARG;
+  cg2d_status_t st = check_params(params);
+  if (st != CG2D_OK) return st;
+  WsLayout L;
+  st = compute_layout(groups, ngroups, params, &L);
+  if (st != CG2D_OK) return st;
+  for (int g = 0; g < ngroups; ++g) {
+    plan[g].on_chip = L.team ? 1 : 0;
+    plan[g].launch = L.team ? g : 0;
+    plan[g].teams = L.team ? L.t[g].nteams : 0;
+    plan[g].ctas_per_team = L.team ? L.t[g].G : 0;
+  }
+  return CG2D_OK;
+}
+
 // checkpoint recording for the exact-mode adjoint (see KParams::ck_r), and where the launch keeps its sums
 struct CkRec {
   double* ck_r;

@@ -1328,9 +1328,13 @@ size_t team_plan(const TopoDev& tp, int count, int nrhs, int mixed, int serial, 
   if (t->nslots > (1ll << 30)) return 0;
   const unsigned es = (mixed ? 4u : 8u) * nrhs;
   // time of a pass in units of an exchange (4.2 us with its fixed steps): 1 + kRowCost per row of the largest CTA's
-  // warps and 32 columns. Measured, LLC90 FP64: 4.6 us at 8 rows a CTA, 9.1 us at 66, 10.6 us at 90. The split with the
-  // least rounds x pass time is taken: 16 solves run 8 teams of 18 CTAs, 64 solves 11 teams of 13.
-  const double steps = (ni + 31) / 32, kRowCost = 0.09;
+  // warps and 32 columns. Measured, LLC90 FP64: 4.6 us at 8 rows a CTA, 9.1 us at 66, 10.6 us at 90. In the FORTRAN order
+  // also a tile's additions: a CTA's n ordered sums run side by side on its warps, at 11.5 + 1.05 n cycles an addition
+  // (latency and shuffles). Measured: 14 cycles with 2 sums, 15 with 4, 19 with 8, 26 with 12 and 14: LLC90 73 us a pass with
+  // 1 tile a CTA, 82 us with 2; LLC32 9.6 us with 1, 23 us with 7. The split with the least rounds x pass time is taken: 16
+  // ROWBLOCK solves run 8 teams of 18 CTAs, 64 run 11 teams of 13; 64 mixed LLC90 solves in the FORTRAN order run 21 teams of
+  // 7 in 4 rounds (14.0 ms for 20 iterations), not 11 teams of 13 in 6 (19.0 ms; 16.3 streamed).
+  const double steps = (ni + 31) / 32, kRowCost = 0.09, kExchangeCycles = 8064.0;
   double best = 0.0;
   size_t best_smem = 0;
   TeamDev cand = *t;
@@ -1384,7 +1388,13 @@ size_t team_plan(const TopoDev& tp, int count, int nrhs, int mixed, int serial, 
     if (o > (size_t)kSmemLimit) continue;
     const int rounds = (count + cand.nteams - 1) / cand.nteams;
     const int per_warp = (max_rows + kTeamWarps - 1) / kTeamWarps;
-    const double cost = rounds * (1.0 + kRowCost * per_warp * steps);
+    double pass = 1.0 + kRowCost * per_warp * steps;
+    if (serial) {
+      const int sums = 2 * nrhs * max_units, turns = (sums + kTeamWarps - 1) / kTeamWarps;
+      const double cycles = 11.5 * turns + 1.05 * sums;
+      pass += (double)ni * nj * cycles / kExchangeCycles;
+    }
+    const double cost = rounds * pass;
     if (best_smem == 0 || cost < best) {
       best = cost;
       best_smem = o;

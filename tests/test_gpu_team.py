@@ -75,3 +75,22 @@ def test_true_residual_in_every_iteration(nrhs):
             (got,) = cg.solve_groups([G], grid_ctas=limit, **kw)
             for (x0, f0, d0), (x1, f1, d1) in zip(ref, got):
                 assert torch.equal(x0, x1) and torch.equal(f0, f1) and torch.equal(d0, d1), limit
+
+
+def test_ordered_sums_count_in_the_split():
+    """64 mixed solves in the FORTRAN order: a pass waits for a tile's ordered additions whatever the team's size, so the
+    split is the one with the fewest rounds (small teams, several tiles a CTA), which the row count alone would not choose.
+    The solves are those of the same instances in other splits bit for bit."""
+    _, _, G = _group(90, 90, 4, 1, 6)
+    G.ops, G.b, G.x0 = (tuple(t.repeat(16, 1, 1, 1) for t in G.ops), [t.repeat(16, 1, 1, 1) for t in G.b],
+                        [t.repeat(16, 1, 1, 1) for t in G.x0])
+    G.norm = G.norm.repeat(16)
+    kw = dict(precision="mixed", sum_order="fortran")
+    (plan,) = cg.solve_plan([G], **kw)
+    assert plan["on_chip"] and plan["teams"] >= 16, plan
+    (((x, f, d),),) = cg.solve_groups([G], **kw)
+    for m in range(1, 16):
+        assert torch.equal(x[:4], x[4 * m:4 * m + 4]) and torch.equal(d[:4], d[4 * m:4 * m + 4])
+    assert not cg.solve_plan([G], grid_ctas=6, **kw)[0]["on_chip"]
+    (((x1, f1, d1),),) = cg.solve_groups([G], grid_ctas=6, **kw)
+    assert torch.equal(x, x1) and torch.equal(f, f1) and torch.equal(d, d1)
