@@ -157,8 +157,9 @@ typedef struct {
 } cg2d_group_plan_t;
 cg2d_status_t cg2d_plan(const cg2d_group_t* groups, int ngroups, const cg2d_params_t* params, cg2d_group_plan_t* plan);
 
-/* Solve every right-hand side of every group: one persistent cooperative launch per group when every group has the
- * same number of right-hand sides and one instance's state fits on chip, else ONE persistent launch for all groups.
+/* Solve every right-hand side of every group in persistent cooperative launches. When every group has the same number of
+ * right-hand sides and one instance's state of each fits on chip, the state stays there: groups that leave the chip idle
+ * share a launch, the others have one each (cg2d_plan tells). Otherwise one launch streams all groups.
  * The workspace (device, >= cg2d_workspace_size bytes, 256-byte aligned) is scratch; it is not
  * read before being written. Returns CG2D_OK when the work was enqueued; per-solve outcomes
  * (convergence, NaN, barrier timeout) are in each solve's diag.status. */

@@ -203,8 +203,8 @@ PROF_SLOTS = len(PROF_NAMES)
 def solve_groups(groups, precision="f64", sum_order="rowblock", rows_per_block=8, replace_every=25,
                  replace_above=100.0, timeout_s=10.0, grid_ctas=0, ctas_per_sm=0, check_status=True,
                  test_missing_arrivals=0, profile=False, unit_deal=0, stages=0, schedule=None):
-    """Run every right-hand side of every group in one call (cg2d_solve_groups): a persistent launch per group while an
-    instance's state fits on chip, else one for all.
+    """Run every right-hand side of every group in one call (cg2d_solve_groups): on chip in one or several persistent
+    launches, or streamed in one (solve_plan tells).
 
     Returns per group a list (one entry per slot) of (x_out, x_fortran or None, diag ndarray of cg2d_diag_t).
     profile=True records per-CTA phase times; they are left in `solve_groups.last_profile` as an array

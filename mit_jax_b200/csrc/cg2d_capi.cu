@@ -60,6 +60,7 @@ struct WsLayout {
   bool team;
   TeamDev t[kMaxGroups];
   size_t t_smem[kMaxGroups], t_zero_end, t_hist, t_coef[kMaxGroups], t_msg[kMaxGroups], t_x[kMaxGroups];
+  int t_last[kMaxGroups];   // the launch that starts with group g runs groups g .. t_last[g] - 1 side by side
 };
 
 int sm_count() {
@@ -142,15 +143,45 @@ cg2d_status_t size_stages(const cg2d_group_t* gr, int ng, int mixed, int serial,
   return CG2D_UNSUPPORTED;
 }
 
-// The launch in teams: taken whenever every group has the same number of right-hand sides and one instance's state fits
+// The launches in teams: taken whenever every group has the same number of right-hand sides and one instance's state fits
 // in the shared memory of the CTAs the launch may use (one per SM, at most grid_ctas). Where both run, the team is faster
 // at every size measured (ms streamed, in teams): LLC32 FORTRAN order 1.8, 0.86; LLC90 FP64 x1 6.9, 2.3; 64 FP64 solves 52,
 // 29; 64 mixed pairs 48, 31; LLC270 FP64 54, 16. What does not fit streams.
+// A group has a launch of its own, on all the CTAs, or shares one with the groups next to it, each on its part of the CTAs.
+// Sharing is for groups bound by latency, which fewer CTAs slow down little: a launch is shared where, by estimate, no group's
+// pass takes more than kShareSlow times as long as alone and the slowest pass at most kShareGain of the passes one after the
+// other. Measured (us for 40 iterations of every group: streamed, one after the other, shared): 4 x LLC8 973, 1250, 409; 2 and
+// 4 x LLC90 FP64 1545, 882, 563 and 2114, 1722, 762; 4 x LLC90 FORTRAN order 9756, 23307, 6257; LLC8 + 16 + 32 + 90 1402,
+// 1392, 518. (With different iteration counts the longest group decides: alone among ended ones, one of 4 x LLC90 takes 8.7 us
+// a pass on its quarter of the chip, 4.6 on all of it, 14 streamed.) Not shared, for want of CTAs: 2 x 16 LLC90 FP64 5665,
+// 3426, -; 2 LLC270 + 8 LLC90 mixed pairs (20 iterations) 5946, 1892, -.
+constexpr double kShareSlow = 1.5, kShareGain = 0.8;
+
+// the parts of `ctas` CTAs that groups a .. b - 1 get in a shared launch: the least each needs, and the rest by their rows;
+// false when they do not fit side by side
+bool share_ctas(const cg2d_group_t* gr, const WsLayout* L, const int* least, int a, int b, int ctas, int* part) {
+  double work[kMaxGroups], all = 0.0;
+  int left = ctas;
+  for (int g = a; g < b; ++g) {
+    left -= least[g];
+    work[g] = (double)gr[g].count * gr[g].topo->nTiles * gr[g].topo->sNy * ((gr[g].topo->sNx + 31) / 32);
+    all += work[g];
+  }
+  if (left < 0) return false;
+  for (int g = a; g < b; ++g) {
+    const long long most = (long long)gr[g].count * L->units[g];   // (a CTA has at least one unit)
+    const long long p = least[g] + (long long)(left * work[g] / all);
+    part[g] = (int)(p < most ? p : most);
+  }
+  return true;
+}
+
 void team_layout(const cg2d_group_t* gr, int ng, const cg2d_params_t* p, WsLayout* L) {
   const bool mixed = p->precision == CG2D_PREC_MIXED, serial = p->sum_order == CG2D_SUM_FORTRAN;
   int ctas = sm_count();
   if (p->grid_ctas > 0 && p->grid_ctas < ctas) ctas = p->grid_ctas;
   L->team = false;
+  double alone[kMaxGroups];
   for (int g = 0; g < ng; ++g) {
     if (gr[g].nrhs != gr[0].nrhs) return;
     TeamDev& t = L->t[g];
@@ -158,8 +189,68 @@ void team_layout(const cg2d_group_t* gr, int ng, const cg2d_params_t* p, WsLayou
     t.nblk = L->nblk[g];
     t.units = L->units[g];
     t.rpb = serial ? gr[g].topo->sNy : L->rpb;
-    L->t_smem[g] = team_plan(topo_dev(gr[g].topo), gr[g].count, gr[g].nrhs, mixed, serial, ctas, &t);
+    L->t_smem[g] = team_plan(topo_dev(gr[g].topo), gr[g].count, gr[g].nrhs, mixed, serial, ctas, &t, &alone[g]);
     if (L->t_smem[g] == 0) return;
+    L->t_last[g] = g + 1;
+  }
+  if (ng > 1) {
+    // the cheapest cut of the groups into launches, by estimate
+    int least[kMaxGroups], part[kMaxGroups];
+    double est[kMaxGroups];
+    bool fits = true;
+    for (int g = 0; g < ng; ++g) {
+      const TopoDev tp = topo_dev(gr[g].topo);
+      least[g] = team_least_ctas(tp, gr[g].nrhs, mixed, serial, L->t[g]);
+      if (least[g] == 0 || least[g] > ctas) { fits = false; break; }
+      est[g] = team_cost(tp, gr[g].count, gr[g].nrhs, serial, least[g], ctas, L->t[g]);
+    }
+    if (fits) {
+      double cost[kMaxGroups + 1];   // of groups 0 .. b - 1
+      int from[kMaxGroups + 1];      // the first group of the launch that ends with group b - 1
+      cost[0] = 0.0;
+      for (int b = 1; b <= ng; ++b) {
+        cost[b] = cost[b - 1] + est[b - 1];
+        from[b] = b - 1;
+        for (int a = b - 2; a >= 0; --a) {
+          if (!share_ctas(gr, L, least, a, b, ctas, part)) break;
+          double slowest = 0.0, sum = 0.0;
+          bool ok = true;
+          for (int g = a; g < b && ok; ++g) {
+            const double c = team_cost(topo_dev(gr[g].topo), gr[g].count, gr[g].nrhs, serial, least[g], part[g], L->t[g]);
+            ok = c <= kShareSlow * est[g];
+            slowest = c > slowest ? c : slowest;
+            sum += est[g];
+          }
+          if (ok && slowest <= kShareGain * sum && cost[a] + slowest < cost[b]) {
+            cost[b] = cost[a] + slowest;
+            from[b] = a;
+          }
+        }
+      }
+      // the splits of the shared launches; one that turns out not to fit or not to pay has its groups one after the other
+      for (int b = ng; b > 0; b = from[b]) {
+        const int a = from[b];
+        if (b - a < 2 || !share_ctas(gr, L, least, a, b, ctas, part)) continue;
+        TeamDev t[kMaxGroups];
+        size_t smem[kMaxGroups];
+        double slowest = 0.0, sum = 0.0;
+        bool ok = true;
+        for (int g = a; g < b && ok; ++g) {
+          double c = 0.0;
+          t[g] = L->t[g];
+          smem[g] = team_plan(topo_dev(gr[g].topo), gr[g].count, gr[g].nrhs, mixed, serial, part[g], &t[g], &c);
+          ok = smem[g] != 0 && c <= kShareSlow * alone[g];
+          slowest = c > slowest ? c : slowest;
+          sum += alone[g];
+        }
+        if (!ok || slowest > kShareGain * sum) continue;
+        for (int g = a; g < b; ++g) {
+          L->t[g] = t[g];
+          L->t_smem[g] = smem[g];
+        }
+        L->t_last[a] = b;
+      }
+    }
   }
   L->team = true;
   size_t o = L->zero_end;
@@ -421,9 +512,14 @@ cg2d_status_t cg2d_plan(const cg2d_group_t* groups, int ngroups, const cg2d_para
   WsLayout L;
   st = compute_layout(groups, ngroups, params, &L);
   if (st != CG2D_OK) return st;
+  int launch = -1, last = 0;
   for (int g = 0; g < ngroups; ++g) {
     plan[g].on_chip = L.team ? 1 : 0;
-    plan[g].launch = L.team ? g : 0;
+    if (L.team && g == last) {
+      ++launch;
+      last = L.t_last[g];
+    }
+    plan[g].launch = L.team ? launch : 0;
     plan[g].teams = L.team ? L.t[g].nteams : 0;
     plan[g].ctas_per_team = L.team ? L.t[g].G : 0;
   }
@@ -440,30 +536,38 @@ struct CkRec {
   int* hist_len;
 };
 
-// the launch of kp's groups in teams (cg2d_team.cu)
+// the launches of kp's groups in teams (cg2d_team.cu)
 static cg2d_status_t launch_in_teams(const KParams& kp, const WsLayout& L, char* ws, cudaStream_t stream) {
   cudaError_t e = cudaMemsetAsync(ws, 0, L.t_zero_end, stream);
-  for (int g = 0; g < kp.ngroups && e == cudaSuccess; ++g) {   // one launch per group
-    TeamParams tp;
-    std::memset(&tp, 0, sizeof(tp));
-    tp.g = kp.g[g];
-    tp.t = L.t[g];
-    tp.t.msg = ws + L.t_msg[g];
-    tp.t.x = reinterpret_cast<double*>(ws + L.t_x[g]);
-    tp.replace_every = kp.replace_every;
-    tp.replace_above = kp.replace_above;
-    tp.hist = kp.hist;
-    tp.hist_len = kp.hist_len;
-    tp.gs = kp.gs;
-    tp.timeout_ns = kp.timeout_ns;
-    tp.test_missing = kp.test_missing;
-    tp.prof = kp.prof;
-    tp.ck_r = kp.ck_r;
-    tp.ck_s = kp.ck_s;
-    tp.ck_stride = kp.ck_stride;
-    tp.ck_every = kp.ck_every;
-    tp.t.coef = ws + L.t_coef[g];
-    e = launch_team(tp, kp.mixed, kp.serial, L.t_smem[g], stream);
+  for (int a = 0; a < kp.ngroups && e == cudaSuccess; a = L.t_last[a]) {
+    TeamGroups kg;
+    std::memset(&kg, 0, sizeof(kg));
+    size_t smem = 0;
+    for (int g = a; g < L.t_last[a]; ++g) {
+      TeamParams& tp = kg.p[kg.n];
+      tp.g = kp.g[g];
+      tp.t = L.t[g];
+      tp.t.msg = ws + L.t_msg[g];
+      tp.t.x = reinterpret_cast<double*>(ws + L.t_x[g]);
+      tp.replace_every = kp.replace_every;
+      tp.replace_above = kp.replace_above;
+      tp.hist = kp.hist;
+      tp.hist_len = kp.hist_len;
+      tp.gs = kp.gs;
+      tp.timeout_ns = kp.timeout_ns;
+      tp.test_missing = kp.test_missing;
+      tp.prof = kp.prof;
+      tp.ck_r = kp.ck_r;
+      tp.ck_s = kp.ck_s;
+      tp.ck_stride = kp.ck_stride;
+      tp.ck_every = kp.ck_every;
+      tp.t.coef = ws + L.t_coef[g];
+      kg.first[kg.n + 1] = kg.first[kg.n] + tp.t.G * tp.t.nteams;
+      ++kg.n;
+      if (L.t_smem[g] > smem) smem = L.t_smem[g];
+    }
+    e = kg.n == 1 ? launch_team(kg.p[0], kp.mixed, kp.serial, smem, stream)
+                  : launch_team_groups(kg, kp.mixed, kp.serial, smem, stream);
   }
   if (e != cudaSuccess) { cudaGetLastError(); return CG2D_CUDA_ERROR; }
   return CG2D_OK;

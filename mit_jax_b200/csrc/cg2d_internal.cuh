@@ -233,6 +233,12 @@ struct TeamParams {   // one group
   int ck_every;
 };
 
+struct TeamGroups {   // groups side by side in one launch: group g's CTAs are first[g] .. first[g + 1] - 1
+  int n;
+  int first[kMaxGroups + 1];
+  TeamParams p[kMaxGroups];
+};
+
 // exact-mode adjoint (cg2d_adjoint.cu)
 struct ExactArgs {
   int batch, max_iters, checkpoint, rows_per_block;
@@ -261,11 +267,16 @@ cudaError_t launch_solver(const KParams& kp, int grid, size_t smem, cudaStream_t
 cudaError_t solver_occupancy(const KParams& kp, size_t smem, int* blocks_per_sm);
 
 // One group's team plan on `ctas` CTAs (one per SM): fills G, nteams, ub and the shared-memory layout of t (its nblk, units, rpb
-// and the group's tp, count, nrhs are set) and returns a CTA's dynamic shared memory, or 0 when no split fits.
-size_t team_plan(const TopoDev& tp, int count, int nrhs, int mixed, int serial, int ctas, TeamDev* t);
+// and the group's tp, count, nrhs are set) and returns a CTA's dynamic shared memory, or 0 when no split fits. cost: rounds x
+// pass time, in units of an exchange.
+size_t team_plan(const TopoDev& tp, int count, int nrhs, int mixed, int serial, int ctas, TeamDev* t, double* cost);
+// The same without the split itself: CTAs of a team that surely fits (0: none), and the cost on `ctas` CTAs at that size or above
+int team_least_ctas(const TopoDev& tp, int nrhs, int mixed, int serial, const TeamDev& t);
+double team_cost(const TopoDev& tp, int count, int nrhs, int serial, int least, int ctas, const TeamDev& t);
 size_t team_msg_bytes(const TopoDev& tp, int nrhs, int mixed, const TeamDev& t);   // per team
 size_t team_coef_bytes(const TopoDev& tp, int mixed, const TeamDev& t);            // per team
 cudaError_t launch_team(const TeamParams& kp, int mixed, int serial, size_t smem, cudaStream_t stream);
+cudaError_t launch_team_groups(const TeamGroups& kg, int mixed, int serial, size_t smem, cudaStream_t stream);
 cudaError_t launch_pack_coef(const GroupDev& g, int mixed, cudaStream_t stream);
 cudaError_t launch_apply_operator(const TopoDev& tp, int batch, double norm, const double* aW, const double* aS,
                                   const double* aC, const double* v, double* out, cudaStream_t stream);

@@ -1237,10 +1237,11 @@ struct Team {
   }
 };
 
+// CTA `cta` of a group's CTAs
 template <bool MIXED, int NS, bool SERIAL, int STEPS>
-__global__ void __launch_bounds__(kTeamThreads, 1) cg2d_team(const __grid_constant__ TeamParams kp) {
+__device__ __forceinline__ void run_team(const TeamParams& kp, int cta) {
   const u64 t_begin = kp.prof && threadIdx.x == 0 ? globaltimer() : 0ull;
-  const int team = blockIdx.x / kp.t.G, rank = blockIdx.x - team * kp.t.G;
+  const int team = cta / kp.t.G, rank = cta - team * kp.t.G;
   Team<MIXED, NS, SERIAL, STEPS> tm(kp, team, rank);
   tm.tables();
   __syncthreads();
@@ -1267,6 +1268,33 @@ __global__ void __launch_bounds__(kTeamThreads, 1) cg2d_team(const __grid_consta
   }
 }
 
+template <bool MIXED, int NS, bool SERIAL, int STEPS>
+__global__ void __launch_bounds__(kTeamThreads, 1) cg2d_team(const __grid_constant__ TeamParams kp) {
+  run_team<MIXED, NS, SERIAL, STEPS>(kp, blockIdx.x);
+}
+
+// Several groups side by side, each on CTAs of its own. Alone, a group that is bound by latency leaves most of the chip idle, and
+// the times of launches one after the other add up: four LLC90 FP64 solves of 40 iterations, one a group, 1722 us as four
+// launches and 762 us as one; in the FORTRAN order 23.3 ms and 6.3 ms. A kernel of its own, because the group's parameters are
+// indexed here and constants of the launch in cg2d_team. (FORTRAN order: the additions bound a pass, so the general row path
+// serves every width.)
+template <bool MIXED, int NS, bool SERIAL>
+__global__ void __launch_bounds__(kTeamThreads, 1) cg2d_team_groups(const __grid_constant__ TeamGroups kg) {
+  int g = 0;
+  while (g + 1 < kg.n && (int)blockIdx.x >= kg.first[g + 1]) ++g;
+  const TeamParams& kp = kg.p[g];
+  const int cta = (int)blockIdx.x - kg.first[g];
+  if constexpr (!SERIAL && (MIXED || NS == 1)) {
+    const int ni = kp.g.tp.ni;
+    if (ni <= 32) run_team<MIXED, NS, SERIAL, 1>(kp, cta);
+    else if (ni <= 64) run_team<MIXED, NS, SERIAL, 2>(kp, cta);
+    else if (ni <= 96) run_team<MIXED, NS, SERIAL, 3>(kp, cta);
+    else run_team<MIXED, NS, SERIAL, 0>(kp, cta);
+  } else {
+    run_team<MIXED, NS, SERIAL, 0>(kp, cta);
+  }
+}
+
 template <bool MIXED, int NS, bool SERIAL>
 const void* team_fn_of(int ni) {
   if constexpr (MIXED || NS == 1) {
@@ -1283,6 +1311,15 @@ const void* team_fn(int mixed, int serial, int nrhs, int ni) {
   }
   if (serial) return nrhs == 2 ? team_fn_of<false, 2, true>(ni) : team_fn_of<false, 1, true>(ni);
   return nrhs == 2 ? team_fn_of<false, 2, false>(ni) : team_fn_of<false, 1, false>(ni);
+}
+
+const void* team_groups_fn(int mixed, int serial, int nrhs) {
+  if (mixed) {
+    if (serial) return nrhs == 2 ? (const void*)cg2d_team_groups<true, 2, true> : (const void*)cg2d_team_groups<true, 1, true>;
+    return nrhs == 2 ? (const void*)cg2d_team_groups<true, 2, false> : (const void*)cg2d_team_groups<true, 1, false>;
+  }
+  if (serial) return nrhs == 2 ? (const void*)cg2d_team_groups<false, 2, true> : (const void*)cg2d_team_groups<false, 1, true>;
+  return nrhs == 2 ? (const void*)cg2d_team_groups<false, 2, false> : (const void*)cg2d_team_groups<false, 1, false>;
 }
 
 // first row of unit u (host)
@@ -1320,21 +1357,56 @@ size_t team_coef_bytes(const TopoDev& tp, int mixed, const TeamDev& t) {
   return (size_t)t.G * 2 * t.max_rows * (tp.ni + 1) * 4 * (mixed ? sizeof(float) : sizeof(double));
 }
 
-size_t team_plan(const TopoDev& tp, int count, int nrhs, int mixed, int serial, int ctas, TeamDev* t) {
+namespace {
+
+// the shared memory of a CTA with at most `rows` rows, `ring` ring rows, `halo` halo cells and `units` units: the layout into c
+size_t smem_layout(const TopoDev& tp, int nrhs, int mixed, int rows, int ring, int halo, int units, TeamDev* c) {
+  const unsigned es = (mixed ? 4u : 8u) * nrhs;
+  const int ni = tp.ni;
+  size_t o = kScalBytes;
+  auto take = [&](size_t bytes) { const size_t p = o; o += (bytes + 127) & ~size_t(127); return (unsigned)p; };
+  c->o_rows = take(sizeof(RowEnt) * (size_t)rows);
+  c->o_halo = take(sizeof(HaloEnt) * (size_t)halo);
+  c->o_send = take(sizeof(SendEnt) * (size_t)halo);   // (at most as many as halo cells)
+  c->o_umsg = take(sizeof(int) * (size_t)c->units);
+  c->o_hval = take((size_t)8 * nrhs * halo);   // (also x at the halo cells, FP64)
+  c->o_units = take(sizeof(int) * ((size_t)units + 1));
+  c->o_rowsum = take(sizeof(double) * (size_t)kTeamKinds * nrhs * rows);
+  c->o_psum = take(sizeof(double) * (size_t)kTeamKinds * nrhs * c->units);
+  c->o_tsum = take(sizeof(double) * (size_t)kTeamKinds * nrhs * tp.T);
+  c->ring_elems = (unsigned)ring * (unsigned)(ni + 2);
+  c->o_r = take((size_t)es * c->ring_elems);
+  c->o_s = take((size_t)es * c->ring_elems);
+  c->o_q = take((size_t)es * rows * ni);
+  return o;
+}
+
+// Time of a pass in units of an exchange (4.2 us with its fixed steps): 1 + kRowCost per row of the largest CTA's warps and
+// 32 columns. Measured, LLC90 FP64: 4.6 us at 8 rows a CTA, 9.1 us at 66, 10.6 us at 90. In the FORTRAN order also a tile's
+// additions: a CTA's n ordered sums run side by side on its warps, at 11.5 + 1.05 n cycles an addition (latency and
+// shuffles). Measured: 14 cycles with 2 sums, 15 with 4, 19 with 8, 26 with 12 and 14: LLC90 73 us a pass with 1 tile a CTA,
+// 82 us with 2; LLC32 9.6 us with 1, 23 us with 7.
+double pass_cost(const TopoDev& tp, int nrhs, int serial, int rows, int units) {
+  const double kRowCost = 0.09, kExchangeCycles = 8064.0, steps = (tp.ni + 31) / 32;
+  double pass = 1.0 + kRowCost * ((rows + kTeamWarps - 1) / kTeamWarps) * steps;
+  if (serial) {
+    const int sums = 2 * nrhs * units, turns = (sums + kTeamWarps - 1) / kTeamWarps;
+    pass += (double)tp.ni * tp.nj * (11.5 * turns + 1.05 * sums) / kExchangeCycles;
+  }
+  return pass;
+}
+
+}  // namespace
+
+size_t team_plan(const TopoDev& tp, int count, int nrhs, int mixed, int serial, int ctas, TeamDev* t, double* cost) {
   if (ctas > kTeamMaxCtas) ctas = kTeamMaxCtas;
   if (t->units > 65535) return 0;
   const int nj = tp.nj, ni = tp.ni, rows = tp.T * nj;
   t->nslots = (2ll * rows + 2ll * t->units * ni + 7) & ~7ll;   // (whole 128-byte lines)
   if (t->nslots > (1ll << 30)) return 0;
-  const unsigned es = (mixed ? 4u : 8u) * nrhs;
-  // time of a pass in units of an exchange (4.2 us with its fixed steps): 1 + kRowCost per row of the largest CTA's
-  // warps and 32 columns. Measured, LLC90 FP64: 4.6 us at 8 rows a CTA, 9.1 us at 66, 10.6 us at 90. In the FORTRAN order
-  // also a tile's additions: a CTA's n ordered sums run side by side on its warps, at 11.5 + 1.05 n cycles an addition
-  // (latency and shuffles). Measured: 14 cycles with 2 sums, 15 with 4, 19 with 8, 26 with 12 and 14: LLC90 73 us a pass with
-  // 1 tile a CTA, 82 us with 2; LLC32 9.6 us with 1, 23 us with 7. The split with the least rounds x pass time is taken: 16
-  // ROWBLOCK solves run 8 teams of 18 CTAs, 64 run 11 teams of 13; 64 mixed LLC90 solves in the FORTRAN order run 21 teams of
-  // 7 in 4 rounds (14.0 ms for 20 iterations), not 11 teams of 13 in 6 (19.0 ms; 16.3 streamed).
-  const double steps = (ni + 31) / 32, kRowCost = 0.09, kExchangeCycles = 8064.0;
+  // The split with the least rounds x pass time is taken: 16 ROWBLOCK solves run 8 teams of 18 CTAs, 64 run 11 teams of 13;
+  // 64 mixed LLC90 solves in the FORTRAN order run 21 teams of 7 in 4 rounds (14.0 ms for 20 iterations), not 11 teams of 13
+  // in 6 (19.0 ms; 16.3 streamed).
   double best = 0.0;
   size_t best_smem = 0;
   TeamDev cand = *t;
@@ -1344,8 +1416,8 @@ size_t team_plan(const TopoDev& tp, int count, int nrhs, int mixed, int serial, 
     if (G > t->units) G = t->units;
     if (G == last_G) continue;   // the same teams, or more of them than fit
     last_G = G;
-    // the smallest largest run
-    int lo = (rows + G - 1) / G, hi = lo + t->rpb + nj;
+    // the smallest largest run (a run leaves less than a unit of its rows unused)
+    int lo = (rows + G - 1) / G, hi = lo + t->rpb - 1;
     unsigned short tmp[kTeamMaxCtas + 2];
     if (lo < 1) lo = 1;
     while (runs_of(cand, nj, hi, G, tmp) > G) hi += nj;
@@ -1370,38 +1442,51 @@ size_t team_plan(const TopoDev& tp, int count, int nrhs, int mixed, int serial, 
     cand.max_rows = max_rows;
     cand.max_units = max_units;
     cand.sum_block = (kTeamKinds * nrhs * max_units + 7) & ~7;   // messages: whole 128-byte lines
-    size_t o = kScalBytes;
-    auto take = [&](size_t bytes) { const size_t p = o; o += (bytes + 127) & ~size_t(127); return (unsigned)p; };
-    cand.o_rows = take(sizeof(RowEnt) * (size_t)max_rows);
-    cand.o_halo = take(sizeof(HaloEnt) * (size_t)max_halo);
-    cand.o_send = take(sizeof(SendEnt) * (size_t)max_halo);   // (at most as many as halo cells)
-    cand.o_umsg = take(sizeof(int) * (size_t)t->units);
-    cand.o_hval = take((size_t)8 * nrhs * max_halo);   // (also x at the halo cells, FP64)
-    cand.o_units = take(sizeof(int) * ((size_t)max_units + 1));
-    cand.o_rowsum = take(sizeof(double) * (size_t)kTeamKinds * nrhs * max_rows);
-    cand.o_psum = take(sizeof(double) * (size_t)kTeamKinds * nrhs * t->units);
-    cand.o_tsum = take(sizeof(double) * (size_t)kTeamKinds * nrhs * tp.T);
-    cand.ring_elems = (unsigned)max_ring * (unsigned)(ni + 2);
-    cand.o_r = take((size_t)es * cand.ring_elems);
-    cand.o_s = take((size_t)es * cand.ring_elems);
-    cand.o_q = take((size_t)es * max_rows * ni);
+    const size_t o = smem_layout(tp, nrhs, mixed, max_rows, max_ring, max_halo, max_units, &cand);
     if (o > (size_t)kSmemLimit) continue;
     const int rounds = (count + cand.nteams - 1) / cand.nteams;
-    const int per_warp = (max_rows + kTeamWarps - 1) / kTeamWarps;
-    double pass = 1.0 + kRowCost * per_warp * steps;
-    if (serial) {
-      const int sums = 2 * nrhs * max_units, turns = (sums + kTeamWarps - 1) / kTeamWarps;
-      const double cycles = 11.5 * turns + 1.05 * sums;
-      pass += (double)ni * nj * cycles / kExchangeCycles;
-    }
-    const double cost = rounds * pass;
-    if (best_smem == 0 || cost < best) {
-      best = cost;
+    const double c = rounds * pass_cost(tp, nrhs, serial, max_rows, max_units);
+    if (best_smem == 0 || c < best) {
+      best = c;
       best_smem = o;
       *t = cand;
     }
   }
+  *cost = best;
   return best_smem;
+}
+
+// (a run of r rows: over at most (r - 2) / nj + 2 tiles; whole tiles in the FORTRAN order)
+int team_least_ctas(const TopoDev& tp, int nrhs, int mixed, int serial, const TeamDev& t) {
+  TeamDev c = t;
+  const int rows = tp.T * tp.nj;
+  auto fits = [&](int r) {
+    const int nseg = serial ? r / tp.nj : (r - 2 + tp.nj) / tp.nj + 1;
+    return smem_layout(tp, nrhs, mixed, r, r + 2 * nseg, 2 * nseg * tp.ni + 2 * r, (r + t.rpb - 1) / t.rpb + nseg, &c) <=
+           (size_t)kSmemLimit;
+  };
+  int lo = 0, hi = (rows + t.rpb - 1) / t.rpb;   // units: lo fit, hi + 1 need not
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) / 2;
+    if (fits(mid * t.rpb)) lo = mid;
+    else hi = mid - 1;
+  }
+  if (lo == 0) return 0;
+  return (t.units + lo - 1) / lo;
+}
+
+double team_cost(const TopoDev& tp, int count, int nrhs, int serial, int least, int ctas, const TeamDev& t) {
+  if (ctas > kTeamMaxCtas) ctas = kTeamMaxCtas;
+  double best = 0.0;
+  for (int nt = 1; nt <= count && nt * least <= ctas; ++nt) {
+    const int G = ctas / nt < t.units ? ctas / nt : t.units;
+    const int units = (t.units + G - 1) / G, nteams = ctas / G < count ? ctas / G : count;
+    int rows = (tp.T * tp.nj + G - 1) / G + (G < t.units ? t.rpb / 2 : 0);   // (runs end at units)
+    if (serial || rows > units * t.rpb) rows = units * t.rpb;
+    const double c = (count + nteams - 1) / nteams * pass_cost(tp, nrhs, serial, rows, units);
+    if (best == 0.0 || c < best) best = c;
+  }
+  return best;
 }
 
 cudaError_t launch_team(const TeamParams& kp, int mixed, int serial, size_t smem, cudaStream_t stream) {
@@ -1413,6 +1498,14 @@ cudaError_t launch_team(const TeamParams& kp, int mixed, int serial, size_t smem
   if (e != cudaSuccess) return e;
   void* args[] = {const_cast<TeamParams*>(&kp)};
   return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kTeamThreads), args, smem, stream);
+}
+
+cudaError_t launch_team_groups(const TeamGroups& kg, int mixed, int serial, size_t smem, cudaStream_t stream) {
+  const void* fn = team_groups_fn(mixed, serial, kg.p[0].g.nrhs);
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);   // (as launch_team)
+  if (e != cudaSuccess) return e;
+  void* args[] = {const_cast<TeamGroups*>(&kg)};
+  return cudaLaunchCooperativeKernel(fn, dim3(kg.first[kg.n]), dim3(kTeamThreads), args, smem, stream);
 }
 
 }  // namespace cg2d

@@ -94,3 +94,51 @@ def test_ordered_sums_count_in_the_split():
     assert not cg.solve_plan([G], grid_ctas=6, **kw)[0]["on_chip"]
     (((x1, f1, d1),),) = cg.solve_groups([G], grid_ctas=6, **kw)
     assert torch.equal(x, x1) and torch.equal(f, f1) and torch.equal(d, d1)
+
+
+GROUPS = [
+    # groups (N, ts, instances), right-hand sides, precision, sum order, launch of each group, CTA limit that streams
+    ([(24, 12, 1), (20, 10, 2), (34, 34, 1)], 1, "f64", "rowblock", [0, 0, 0], 1),
+    ([(90, 90, 1), (90, 90, 1)], 1, "f64", "rowblock", [0, 0], 4),
+    ([(32, 32, 1), (64, 64, 1), (90, 90, 1), (98, 98, 1)], 2, "mixed", "rowblock", [0, 0, 0, 0], 2),
+    ([(64, 64, 1), (98, 98, 1)], 1, "mixed", "rowblock", [0, 0], 2),
+    ([(30, 30, 1), (20, 10, 1)], 2, "f64", "rowblock", [0, 0], 1),
+    ([(32, 32, 1), (8, 8, 2), (16, 8, 1), (40, 40, 1)], 1, "f64", "fortran", [0, 0, 0, 0], 1),
+    ([(24, 24, 1), (32, 32, 1)], 2, "f64", "fortran", [0, 0], 1),
+    ([(48, 48, 1), (24, 24, 2)], 2, "mixed", "fortran", [0, 0], 1),
+    ([(48, 48, 1), (60, 60, 1)], 1, "mixed", "fortran", [0, 0], 1),
+    ([(90, 90, 4), (90, 90, 4), (90, 90, 4)], 1, "f64", "fortran", [0, 0, 1], 8),
+    ([(90, 90, 11), (90, 90, 11)], 1, "f64", "rowblock", [0, 1], 8),
+]
+
+
+@pytest.mark.parametrize("sizes,nrhs,precision,order,launches,streams", GROUPS)
+def test_groups_share_a_launch(sizes, nrhs, precision, order, launches, streams):
+    """Several groups in one call: side by side in one launch, one after the other, and streamed, equal bit for bit; the plan
+    says which groups share a launch."""
+    groups = [_group(N, ts, count, nrhs, 15 + 10 * i)[2] for i, (N, ts, count) in enumerate(sizes)]
+    kw = dict(precision=precision, sum_order=order)
+    plan = cg.solve_plan(groups, **kw)
+    assert all(p["on_chip"] for p in plan) and [p["launch"] for p in plan] == launches, plan
+    assert not any(p["on_chip"] for p in cg.solve_plan(groups, grid_ctas=streams, **kw))
+    res, ref = cg.solve_groups(groups, **kw), cg.solve_groups(groups, grid_ctas=streams, **kw)
+    for slots, ref_slots in zip(res, ref):
+        for (x0, f0, d0), (x1, f1, d1) in zip(ref_slots, slots):
+            assert torch.equal(x0, x1) and torch.equal(f0, f1) and torch.equal(d0, d1)
+    if precision == "f64":   # (mixed groups of several and of one have other row blocks)
+        for G, slots in zip(groups, res):
+            (alone,) = cg.solve_groups([G], **kw)
+            for (x0, f0, d0), (x1, f1, d1) in zip(alone, slots):
+                assert torch.equal(x0, x1) and torch.equal(f0, f1) and torch.equal(d0, d1)
+
+
+def test_time_limit_in_a_shared_launch():
+    """A wait that cannot complete runs out in every group of a shared launch, and the next solve is fine."""
+    groups = [_group(N, N, 2, 1, 20)[2] for N in (8, 16)]
+    assert [p["launch"] for p in cg.solve_plan(groups)] == [0, 0]
+    res = cg.solve_groups(groups, timeout_s=0.2, check_status=False, test_missing_arrivals=1)
+    for ((_, _, dg),) in res:
+        assert all(r["status"] == "barrier_timeout" for r in cg.diag_records(dg))
+    ref = cg.solve_groups(groups, grid_ctas=1)
+    for ((x0, _, d0),), ((x1, _, d1),) in zip(ref, cg.solve_groups(groups)):
+        assert torch.equal(x0, x1) and torch.equal(d0, d1)
