@@ -144,7 +144,7 @@ typedef struct {
 
 void cg2d_default_params(cg2d_params_t* p);
 
-/* Bytes of device workspace a cg2d_solve_groups call with these groups needs. */
+/* Bytes of device workspace for a cg2d_solve_groups call with these groups. */
 size_t cg2d_workspace_size(const cg2d_group_t* groups, int ngroups, const cg2d_params_t* params);
 
 /* How a cg2d_solve_groups call with these groups and parameters would run (sizes and parameters decide; nothing is

@@ -47,7 +47,7 @@ TopoDev topo_dev(const cg2d_topology* tp) {
 }
 
 struct WsLayout {
-  size_t gs, rmax, prof, zero_end, hist, part, total;
+  size_t gs, rmax, prof, zero_end, hist, part, total, stream_total;   // stream_total: what the streaming launch needs
   size_t vec[kMaxGroups], cpk[kMaxGroups];
   long long vec_stride[kMaxGroups];
   long long vec_off[kMaxGroups][V_NVEC];
@@ -348,7 +348,7 @@ cg2d_status_t compute_layout(const cg2d_group_t* gr, int ng, const cg2d_params_t
     L->cpk[g] = o;
     o += al(vsz * 2 * (size_t)tp->nTiles * (tp->sNy + 1) * 3 * coef_pitch(tp->sNx) * gr[g].count);
   }
-  L->total = o;
+  L->total = L->stream_total = o;
   team_layout(gr, ng, p, L);
   return CG2D_OK;
 }
@@ -526,6 +526,16 @@ cg2d_status_t cg2d_plan(const cg2d_group_t* groups, int ngroups, const cg2d_para
   return CG2D_OK;
 }
 
+// the least workspace a call is accepted with: cg2d_workspace_size, or a little less where the teams need more than the
+// streaming launch (which then runs)
+static size_t least_workspace(const cg2d_group_t* groups, int ngroups, const cg2d_params_t* params) {
+  cg2d_params_t def;
+  if (!params) { cg2d_default_params(&def); params = &def; }
+  WsLayout L;
+  if (check_params(params) != CG2D_OK || compute_layout(groups, ngroups, params, &L) != CG2D_OK) return 0;
+  return L.stream_total;
+}
+
 // checkpoint recording for the exact-mode adjoint (see KParams::ck_r), and where the launch keeps its sums
 struct CkRec {
   double* ck_r;
@@ -585,7 +595,8 @@ static cg2d_status_t solve_groups_impl(const cg2d_group_t* groups, int ngroups, 
   st = compute_layout(groups, ngroups, params, &L);
   if (st != CG2D_OK) return st;
   if (!workspace || (reinterpret_cast<uintptr_t>(workspace) % kAlign) != 0) return CG2D_BAD_ARG;
-  if (workspace_bytes < L.total) return CG2D_WORKSPACE_TOO_SMALL;
+  if (workspace_bytes < L.stream_total) return CG2D_WORKSPACE_TOO_SMALL;
+  if (workspace_bytes < L.total) L.team = false;   // (total is above stream_total only where the teams need more)
   for (int g = 0; g < ngroups; ++g) {
     const cg2d_group_t& G = groups[g];
     if (!G.aW2d || !G.aS2d || !G.aC2d || !G.pW || !G.pS || !G.pC) return CG2D_BAD_ARG;
@@ -781,13 +792,14 @@ cg2d_status_t cg2d_adjoint_ecco(const cg2d_topology_t* topo, int batch, double c
   if (!topo || batch < 1 || !x_bar || !lam || !diag || !workspace || (coeff_grad && (!x || !gW || !gS || !gC)) ||
       coeff_grad < 0 || coeff_grad > 1)
     return CG2D_BAD_ARG;
-  const size_t need = cg2d_adjoint_ecco_workspace_size(topo, batch, adj_max_iters, params);
-  if (need == 0) return CG2D_BAD_ARG;
-  if (workspace_bytes < need) return CG2D_WORKSPACE_TOO_SMALL;
   cg2d_group_t g = one_group(topo, batch, adj_tolerance, adj_max_iters);
-  const size_t solver = round256(cg2d_workspace_size(&g, 1, params));
+  const size_t least = least_workspace(&g, 1, params);
+  if (least == 0) return CG2D_BAD_ARG;
   const TopoDev tp = topo_dev(topo);
   const size_t vb = sizeof(double) * (size_t)batch * tp.T * tp.npy * tp.npx;
+  if (workspace_bytes < round256(least) + vb) return CG2D_WORKSPACE_TOO_SMALL;
+  // the solver's workspace, then the zero first guess
+  const size_t solver = (workspace_bytes - vb) & ~size_t(255);
   double* zero = reinterpret_cast<double*>(static_cast<char*>(workspace) + solver);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (cudaMemsetAsync(zero, 0, vb, st) != cudaSuccess) { cudaGetLastError(); return CG2D_CUDA_ERROR; }
@@ -886,15 +898,17 @@ cg2d_status_t cg2d_solve_exact(const cg2d_topology_t* topo, int batch, double cg
   if (!topo || batch < 1 || max_iters < 0 || checkpoint_every < 0 || rows_per_block < 8 || !x_bar || !x_out ||
       !diag || !b_bar || !gW || !gS || !gC || !gpW || !gpS || !gpC || !workspace)
     return CG2D_BAD_ARG;
-  const size_t need = cg2d_solve_exact_workspace_size(topo, batch, max_iters, rows_per_block, checkpoint_every);
-  if (need == 0) return CG2D_BAD_ARG;
-  if (workspace_bytes < need) return CG2D_WORKSPACE_TOO_SMALL;
-  if ((reinterpret_cast<uintptr_t>(workspace) % kAlign) != 0) return CG2D_BAD_ARG;
-  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
+  const cg2d_params_t p = exact_params(rows_per_block);
+  cg2d_group_t g = one_group(topo, batch, tolerance, max_iters);
+  const size_t least = least_workspace(&g, 1, &p);
+  if (least == 0) return CG2D_BAD_ARG;
   const TopoDev tp = topo_dev(topo);
   // workspace: the adjoint's (its checkpoint blocks receive the forward's r_c, s_{c-1}), then the solver's
   char* adj = static_cast<char*>(workspace);
   const size_t adj_bytes = round256(exact_adjoint_workspace(tp, batch, max_iters, checkpoint_every));
+  if (workspace_bytes < adj_bytes + least) return CG2D_WORKSPACE_TOO_SMALL;
+  if ((reinterpret_cast<uintptr_t>(workspace) % kAlign) != 0) return CG2D_BAD_ARG;
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   CkRec ck;
   exact_checkpoints(tp, batch, max_iters, checkpoint_every, adj, &ck.ck_r, &ck.ck_s, &ck.stride);
   ck.every = checkpoint_every > 0 ? checkpoint_every : (max_iters > 0 ? max_iters : 1);
@@ -902,8 +916,6 @@ cg2d_status_t cg2d_solve_exact(const cg2d_topology_t* topo, int batch, double cg
   int hist_len = 0;
   ck.hist = &hist;
   ck.hist_len = &hist_len;
-  const cg2d_params_t p = exact_params(rows_per_block);
-  cg2d_group_t g = one_group(topo, batch, tolerance, max_iters);
   g.aW2d = aW2d; g.aS2d = aS2d; g.aC2d = aC2d; g.pW = pW; g.pS = pS; g.pC = pC;
   g.cg2dNorm = cg2dNorm;
   g.cg2dNorm_per_instance = cg2dNorm_per_instance;
@@ -1162,10 +1174,10 @@ cg2d_status_t cg2d_solve_f64_noalloc(const cg2d_topology_t* topo, int batch, dou
   g.diag[0] = diag;
   g.tolerance[0] = tolerance;
   g.max_iters[0] = max_iters;
-  // the workspace this solve needs must fit the fixed array
   // phase profiles would be written into the hidden array, where no caller can read them back
   if (params && params->profile) return CG2D_BAD_ARG;
-  const size_t need = cg2d_workspace_size(&g, 1, params);
+  // the workspace this solve needs at least must fit the fixed array
+  const size_t need = least_workspace(&g, 1, params);
   // arguments the solver rejects: the same status as cg2d_solve_f64 (the checks run before the workspace is used)
   if (need == 0) return cg2d_solve_groups(&g, 1, params, nullptr, 0, stream);
   if (need > (size_t)CG2D_NOALLOC_SCRATCH_BYTES) return CG2D_WORKSPACE_TOO_SMALL;

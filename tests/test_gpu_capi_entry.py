@@ -96,3 +96,49 @@ def test_adjoint_ecco_entry_equals_autograd(problem, coeff_grad):
             torch.testing.assert_close(g, a.grad, rtol=0, atol=0)
         else:
             assert a.grad is None and not g.any()
+
+
+def test_workspace_of_the_streaming_launch_is_accepted():
+    """Teams of CTAs can need a little more workspace than the streaming launch (here: mixed, 52 tiles of 16 points). A call
+    that brings only what the streaming launch needs is not refused: it streams, with the same result bit for bit."""
+    from mit_jax_b200.synthetic import LLCSynthetic
+    syn = LLCSynthetic(32, 16, 4)
+    ops1, norm = syn.operator()
+    dev = torch.device("cuda")
+    ops = tuple(torch.as_tensor(np.ascontiguousarray(a)).to(dev)[None] for a in ops1)
+    b = torch.as_tensor(np.ascontiguousarray(syn.rhs())).to(dev)[None]
+    x0 = torch.zeros_like(b)
+    ex = cg.default_exchanger(syn.L)
+    L, h, stream = capi.lib(), ex.handle(dev), torch.cuda.current_stream().cuda_stream
+    params, small = capi.default_params(), capi.default_params()
+    params.precision = small.precision = capi.PREC_MIXED
+    small.grid_ctas = 1
+    G = cg.GroupSpec(ex, ops, [b], [x0], [1e-9], [200], float(norm))
+    assert cg.solve_plan([G], precision="mixed")[0]["on_chip"]
+    assert not cg.solve_plan([G], precision="mixed", grid_ctas=1)[0]["on_chip"]
+    g = capi.Group()
+    g.topo, g.count, g.nrhs = h, 1, 1
+    g.max_iters[0], g.tolerance[0] = 200, 1e-9
+    need, least = (L.cg2d_workspace_size(ctypes.byref(g), 1, ctypes.byref(p)) for p in (params, small))
+    assert 0 < least < need
+    ws = torch.empty(need + 256 + 8 * b.numel() + 256, dtype=torch.uint8, device=dev)
+    base = ws.data_ptr() + (-ws.data_ptr()) % 256
+    out = []
+    for nbytes, status in ((need, capi.CG2D_OK), (least, capi.CG2D_OK), (least - 8, capi.CG2D_WORKSPACE_TOO_SMALL)):
+        x, xf = torch.empty_like(b), torch.empty_like(b)
+        dg = torch.zeros((1, capi.DIAG_BYTES), dtype=torch.uint8, device=dev)
+        assert L.cg2d_solve_mixed(h, 1, float(norm), *(_p(t) for t in ops), _p(b), _p(x0), 1e-9, 200, _p(x), _p(xf), _p(dg),
+                                  ctypes.byref(params), base, nbytes, stream) == status
+        if status == capi.CG2D_OK:
+            torch.cuda.synchronize()
+            out.append((x, xf, dg))
+    assert all(torch.equal(a, c) for a, c in zip(*out))
+    full = L.cg2d_adjoint_ecco_workspace_size(h, 1, 200, ctypes.byref(params))
+    lam = []
+    for nbytes in (full, full - (need - least) // 256 * 256):
+        lm, dg = torch.empty_like(b), torch.zeros((1, capi.DIAG_BYTES), dtype=torch.uint8, device=dev)
+        assert L.cg2d_adjoint_ecco(h, 1, float(norm), None, *(_p(t) for t in ops), None, _p(b), 1e-9, 200, 0, _p(lm), None,
+                                   None, None, _p(dg), ctypes.byref(params), base, nbytes, stream) == capi.CG2D_OK
+        torch.cuda.synchronize()
+        lam.append(lm)
+    assert torch.equal(*lam) and torch.equal(lam[0], out[0][0])
