@@ -1239,7 +1239,7 @@ struct Team {
 
 // CTA `cta` of a group's CTAs
 template <bool MIXED, int NS, bool SERIAL, int STEPS>
-__device__ __forceinline__ void run_team(const TeamParams& kp, int cta) {
+__device__ __forceinline__ void run_team(const TeamParams& kp, unsigned cta) {
   const u64 t_begin = kp.prof && threadIdx.x == 0 ? globaltimer() : 0ull;
   const int team = cta / kp.t.G, rank = cta - team * kp.t.G;
   Team<MIXED, NS, SERIAL, STEPS> tm(kp, team, rank);
@@ -1283,7 +1283,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) cg2d_team_groups(const __grid
   int g = 0;
   while (g + 1 < kg.n && (int)blockIdx.x >= kg.first[g + 1]) ++g;
   const TeamParams& kp = kg.p[g];
-  const int cta = (int)blockIdx.x - kg.first[g];
+  const unsigned cta = blockIdx.x - kg.first[g];
   if constexpr (!SERIAL && (MIXED || NS == 1)) {
     const int ni = kp.g.tp.ni;
     if (ni <= 32) run_team<MIXED, NS, SERIAL, 1>(kp, cta);
