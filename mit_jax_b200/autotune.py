@@ -1,20 +1,20 @@
-"""Launch-schedule autotuner for the persistent CG2D launch (cg2d_solve_groups).
+"""Launch-schedule autotuner for cg2d_solve_groups.
 
 A schedule says where the work runs, not what it computes:
-- grid_ctas: how many CTAs the cooperative launch has;
-- ctas_per_sm: how many of them share an SM (1, or the occupancy maximum);
-- unit_deal: how the work units (instance, tile, row block) are dealt to them, round-robin (0) or in contiguous
-  runs (1);
-- stages: the depth of each CTA's copy pipeline (2 to 4 stage buffers; deeper takes more shared memory).
+- grid_ctas: how many CTAs the launch may have;
+- ctas_per_sm, unit_deal, stages: streaming launch only. How many CTAs share an SM (1, or the occupancy maximum), how the
+  work units (instance, tile, row block) are dealt to the CTAs, round-robin (0) or in contiguous runs (1), and the depth
+  of each CTA's copy pipeline (2 to 4 stage buffers; deeper takes more shared memory).
+Solves whose state stays on chip split themselves over the CTAs they may use, so only grid_ctas changes their launch.
 No schedule changes a result bit: every sum is formed from per-unit partials in one fixed order, whichever CTA
 computed a unit (the GPU tests solve every candidate and compare them bit for bit).
 
 `tune` times every candidate on the caller's own groups with a fixed iteration count (tolerance 0 and `iters`
 iterations per right-hand side, so that every candidate does the same work and the per-iteration cost decides),
-keeps the fastest, and caches it per workload signature: device name and SM count, precision, sum order,
-ROWBLOCK height, residual-replacement settings, and per group (tiles, sNy, sNx, count, right-hand sides). The
-cache lives in this process; with MIT_JAX_B200_TUNE_CACHE set to a file path it is also read from and written
-to that JSON file.
+keeps the fastest, and caches it per workload signature: kernel generation, device name and SM count, precision, sum
+order, ROWBLOCK height, residual-replacement settings, and per group (tiles, sNy, sNx, count, right-hand sides).
+The cache lives in this process; with
+MIT_JAX_B200_TUNE_CACHE set to a file path it is also read from and written to that JSON file.
 """
 
 import json
@@ -22,6 +22,10 @@ import os
 import threading
 
 import torch
+
+# Part of the cache key: raised when a kernel or its route changes, so that a cached schedule of other kernels is not used.
+# (1, without a key: every solve streamed. 2: solves that fit stay on chip, where a reduced grid only takes CTAs away.)
+KERNELS = 2
 
 _CACHE = {}
 _LOCK = threading.Lock()
@@ -37,7 +41,7 @@ def signature(groups, *, precision, sum_order, rows_per_block, replace_every=25,
     for G in groups:
         L = G.ex.L
         shapes.append([int(L.nTiles), int(L.sNy), int(L.sNx), int(G.b[0].shape[0]), len(G.b)])
-    key = {"device": props.name, "sms": int(props.multi_processor_count), "precision": precision,
+    key = {"kernels": KERNELS, "device": props.name, "sms": int(props.multi_processor_count), "precision": precision,
            "sum_order": sum_order, "rows_per_block": int(rows_per_block), "groups": shapes}
     if precision == "mixed":
         key["replace"] = [int(replace_every), float(replace_above)]

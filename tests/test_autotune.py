@@ -1,6 +1,9 @@
 """The autotuner's host side (no GPU): the candidate schedules and the JSON cache."""
 
 import json
+from types import SimpleNamespace
+
+import torch
 
 from mit_jax_b200 import autotune
 
@@ -35,3 +38,19 @@ def test_cache_file_round_trip(tmp_path, monkeypatch):
     monkeypatch.setattr(autotune, "_CACHE", {})
     monkeypatch.setattr(autotune, "_LOADED", set())
     assert autotune.cached("bad") is None
+
+
+def test_schedules_of_other_kernels_are_not_reused(monkeypatch):
+    """A schedule cached for the kernels of before (a reduced grid can win among streaming launches; on chip it only takes
+    CTAs away) has another key, also when it came from a cache file."""
+    props = SimpleNamespace(name="GPU", multi_processor_count=148)
+    monkeypatch.setattr(torch.cuda, "get_device_properties", lambda dev: props)
+    G = SimpleNamespace(ex=SimpleNamespace(L=SimpleNamespace(nTiles=13, sNy=90, sNx=90)), b=[torch.zeros(4, 1)])
+    kw = dict(precision="f64", sum_order="rowblock", rows_per_block=8)
+    before = json.dumps({"device": "GPU", "sms": 148, "precision": "f64", "sum_order": "rowblock", "rows_per_block": 8,
+                         "groups": [[13, 90, 90, 4, 1]]}, sort_keys=True)
+    monkeypatch.setattr(autotune, "_CACHE", {before: {"grid_ctas": 74, "ctas_per_sm": 1, "unit_deal": 0, "stages": 2}})
+    key = autotune.signature([G], **kw)
+    assert autotune.cached(before) is not None and autotune.cached(key) is None
+    monkeypatch.setattr(autotune, "KERNELS", autotune.KERNELS + 1)
+    assert autotune.signature([G], **kw) != key
