@@ -13,7 +13,7 @@ computed a unit (the GPU tests solve every candidate and compare them bit for bi
 iterations per right-hand side, so that every candidate does the same work and the per-iteration cost decides),
 keeps the fastest, and caches it per workload signature: kernel generation, device name and SM count, precision, sum
 order, ROWBLOCK height, residual-replacement settings, and per group (tiles, sNy, sNx, count, right-hand sides).
-The cache lives in this process; with
+Candidates that come out as the same launch (cg2d_plan) are timed once. The cache lives in this process; with
 MIT_JAX_B200_TUNE_CACHE set to a file path it is also read from and written to that JSON file.
 """
 
@@ -102,9 +102,9 @@ def cached(key):
 def tune(groups, *, precision="f64", sum_order="rowblock", rows_per_block=8, replace_every=25,
          replace_above=100.0, iters=20, reps=3, force=False, report=None):
     """The fastest schedule for these groups (a dict of grid_ctas, ctas_per_sm, unit_deal, stages), from the cache or by
-    timing every candidate. report, if a list, receives one (schedule, milliseconds or None) per candidate."""
+    timing every distinct launch. report, if a list, receives one (schedule, milliseconds or None) per candidate."""
     from mit_jax_b200 import capi
-    from mit_jax_b200.cg2d import GroupSpec, solve_groups
+    from mit_jax_b200.cg2d import GroupSpec, solve_groups, solve_plan
 
     dev = groups[0].b[0].device
     key = signature(groups, precision=precision, sum_order=sum_order, rows_per_block=rows_per_block,
@@ -119,8 +119,16 @@ def tune(groups, *, precision="f64", sum_order="rowblock", rows_per_block=8, rep
     stream = torch.cuda.current_stream(dev)
     sms = torch.cuda.get_device_properties(dev).multi_processor_count
     best, best_ms = None, None
+    timed = {}
     for cand in candidates(sms):
+        launch = None
         try:
+            plan = solve_plan(proxy, precision=precision, sum_order=sum_order, rows_per_block=rows_per_block, **cand)
+            launch = str(plan) if all(p["on_chip"] for p in plan) else str(cand)
+            if launch in timed:
+                if report is not None:
+                    report.append((dict(cand), timed[launch]))
+                continue
             solve_groups(proxy, **kw, **cand)                      # warm-up, and rejects unsupported launches
             torch.cuda.synchronize(dev)
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -134,6 +142,7 @@ def tune(groups, *, precision="f64", sum_order="rowblock", rows_per_block=8, rep
             ms = sorted(times)[len(times) // 2]
         except capi.Cg2dError:
             ms = None
+        timed[launch] = ms
         if report is not None:
             report.append((dict(cand), ms))
         if ms is not None and (best_ms is None or ms < best_ms):

@@ -83,6 +83,34 @@ def test_tune_picks_a_candidate_and_caches_it(workload, monkeypatch):
     _same(cg.solve_groups([G], precision="mixed"), cg.solve_groups([G], precision="mixed", schedule="auto"))
 
 
+@pytest.mark.parametrize("route", ["on_chip", "streamed"])
+def test_tune_times_each_distinct_launch_once(workload, route, monkeypatch):
+    """On chip only grid_ctas changes the launch, so at most one launch per CTA count is timed; a workload that streams has
+    every candidate timed."""
+    _, G = workload
+    monkeypatch.delenv("MIT_JAX_B200_TUNE_CACHE", raising=False)
+    monkeypatch.setattr(autotune, "_CACHE", {})
+    groups = [G]
+    if route == "streamed":   # groups with different numbers of right-hand sides
+        groups = [G, cg.GroupSpec(G.ex, G.ops, G.b[:1], G.x0[:1], G.tol[:1], G.max_iters[:1], G.norm)]
+    seen, solve, report = [], cg.solve_groups, []
+
+    def counting(groups, **kw):
+        seen.append((kw["grid_ctas"], kw["ctas_per_sm"], kw["unit_deal"], kw["stages"]))
+        return solve(groups, **kw)
+
+    monkeypatch.setattr(cg, "solve_groups", counting)
+    autotune.tune(groups, precision="mixed", iters=3, reps=1, report=report)
+    cands = autotune.candidates(torch.cuda.get_device_properties(0).multi_processor_count)
+    on_chip = [all(p["on_chip"] for p in cg.solve_plan(groups, precision="mixed", **c)) for c in cands]
+    assert all(on_chip) if route == "on_chip" else not any(on_chip)
+    assert [c for c, _ in report] == cands
+    if route == "on_chip":
+        assert len(set(seen)) <= len({min(c["grid_ctas"], 148) for c in cands})
+    else:
+        assert len(set(seen)) == len(cands)
+
+
 def test_graph_replay_equals_eager_on_new_inputs(workload):
     ex, G = workload
     norms = G.norm
