@@ -1,6 +1,7 @@
 """Launch schedules and CUDA-graph replay on the GPU. Every schedule the autotuner can pick (CTA count, CTAs per
-SM, unit deal) gives the same solutions and diagnostics bit for bit, in FP64 and in mixed precision; the tuner
-returns one of them and caches it; schedule="auto" solves like the default; and a captured launch replayed with
+SM, unit deal) gives the same solutions and diagnostics bit for bit, in FP64 and in mixed precision (these solves stay on
+chip, where only the CTA count changes the launch; tests/test_gpu_streaming.py has the schedules of the streaming kernel);
+the tuner returns one of them and caches it; schedule="auto" solves like the default; and a captured launch replayed with
 new inputs written into its static tensors equals the eager solve of those inputs."""
 
 import pytest
@@ -54,9 +55,8 @@ def test_every_candidate_schedule_is_bitwise_equal(workload, precision):
 
 
 def test_fp64_builds_for_one_and_two_ctas_per_sm_are_bitwise_equal():
-    """One right-hand side, batch 8 LLC90 (1248 work units, at least 8 per SM): the default launch takes the FP64
-    build for 2 CTAs per SM (96 registers a thread), ctas_per_sm 1 the build for one CTA per SM and ctas_per_sm 2
-    the first again. Solutions and diagnostics are the same bit for bit."""
+    """One right-hand side, batch 8 LLC90 (1248 work units, at least 8 per SM), which stays on chip: ctas_per_sm does not
+    change the solve. Where it streams, ctas_per_sm picks the FP64 build (tests/test_gpu_streaming.py)."""
     syn, B = make_batch(90, 8)
     dev = torch.device("cuda")
     ex = cg.default_exchanger(syn.L)

@@ -193,8 +193,9 @@ def test_two_rhs_share_the_operator():
 
 
 def test_mixed_size_groups_llc270_and_llc90():
-    """LLC270 and LLC90 instances in one MIXED launch (two groups): each converges and lies within 1e-11 of the
-    FP64 solve of the same instance (the same two groups in one FP64 launch); the LLC90 iteration counts are within
+    """LLC270 and LLC90 instances in one MIXED call (two groups, on chip; tests/test_gpu_streaming.py has the streamed
+    launch): each converges and lies within 1e-11 of the
+    FP64 solve of the same instance (the same two groups in one FP64 call); the LLC90 iteration counts are within
     5 of the mixed oracle's."""
     from mit_jax_b200.synthetic import LLCSynthetic
     dev = torch.device("cuda")
@@ -257,8 +258,8 @@ def test_operator_symmetric():
 
 
 def test_barrier_time_limit_reports_status():
-    """A grid-wide wait that can never complete (one arrival more than there are CTAs) runs out after the time
-    limit; every solve reports barrier_timeout and the context stays usable."""
+    """A wait that can never complete (on chip: for a message that nobody sends) runs out after the time limit; every solve
+    reports barrier_timeout and the context stays usable."""
     c = load("llc8")
     ex = _ex(c)
     dev = torch.device("cuda")

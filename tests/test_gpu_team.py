@@ -14,18 +14,18 @@ from oracle import cg2d_oracle as O
 pytestmark = pytest.mark.gpu
 
 CASES = [
-    # N, ts, instances, right-hand sides, precision, sum order, rows per block, CTA limits
-    (8, 8, 1, 1, "f64", "rowblock", 8, (1, 5, 13)),
-    (8, 2, 1, 2, "f64", "fortran", 8, (1, 7, 148)),
-    (20, 10, 3, 1, "f64", "rowblock", 8, (1, 2, 17, 148)),
-    (34, 34, 2, 1, "f64", "rowblock", 16, (2, 9, 148)),
-    (36, 12, 5, 2, "mixed", "rowblock", 8, (3, 40, 148)),
-    (66, 66, 2, 1, "mixed", "rowblock", 8, (4, 30, 148)),
-    (90, 90, 3, 2, "mixed", "rowblock", 8, (4, 26, 148)),
-    (90, 90, 2, 1, "f64", "fortran", 8, (4, 13, 148)),
-    (98, 98, 1, 2, "f64", "rowblock", 24, (4, 100, 148)),
-    (130, 130, 1, 1, "mixed", "fortran", 8, (4, 60, 148)),
-    (194, 194, 1, 1, "f64", "rowblock", 8, (4, 90, 148)),
+    # N, ts, instances, right-hand sides, precision, sum order, rows per block, CTA limits, those that stream
+    (8, 8, 1, 1, "f64", "rowblock", 8, (1, 5, 13), ()),
+    (8, 2, 1, 2, "f64", "fortran", 8, (1, 7, 148), ()),
+    (20, 10, 3, 1, "f64", "rowblock", 8, (1, 2, 17, 148), (1,)),
+    (34, 34, 2, 1, "f64", "rowblock", 16, (2, 9, 148), ()),
+    (36, 12, 5, 2, "mixed", "rowblock", 8, (3, 40, 148), (3,)),
+    (66, 66, 2, 1, "mixed", "rowblock", 8, (4, 30, 148), ()),
+    (90, 90, 3, 2, "mixed", "rowblock", 8, (4, 26, 148), (4,)),
+    (90, 90, 2, 1, "f64", "fortran", 8, (4, 13, 148), (4,)),
+    (98, 98, 1, 2, "f64", "rowblock", 24, (4, 100, 148), (4,)),
+    (130, 130, 1, 1, "mixed", "fortran", 8, (4, 60, 148), (4,)),
+    (194, 194, 1, 1, "f64", "rowblock", 8, (4, 90, 148), (4,)),
 ]
 
 
@@ -38,12 +38,14 @@ def _group(N, ts, count, nrhs, iters):
                                 [1e-9, 1e-6][:nrhs], [iters, iters][:nrhs], t["cg2dNorm"], x_fortran=True)
 
 
-@pytest.mark.parametrize("N,ts,count,nrhs,precision,order,rows,limits", CASES)
-def test_every_split_is_bitwise_equal(N, ts, count, nrhs, precision, order, rows, limits):
+@pytest.mark.parametrize("N,ts,count,nrhs,precision,order,rows,limits,streams", CASES)
+def test_every_split_is_bitwise_equal(N, ts, count, nrhs, precision, order, rows, limits, streams):
     _, _, G = _group(N, ts, count, nrhs, 70)
     kw = dict(precision=precision, sum_order=order, rows_per_block=rows)
+    assert cg.solve_plan([G], **kw)[0]["on_chip"]
     (ref,) = cg.solve_groups([G], **kw)
     for limit in limits:
+        assert cg.solve_plan([G], grid_ctas=limit, **kw)[0]["on_chip"] == (limit not in streams), limit
         (got,) = cg.solve_groups([G], grid_ctas=limit, **kw)
         for (x0, f0, d0), (x1, f1, d1) in zip(ref, got):
             assert torch.equal(x0, x1) and torch.equal(f0, f1) and torch.equal(d0, d1), limit
@@ -51,6 +53,8 @@ def test_every_split_is_bitwise_equal(N, ts, count, nrhs, precision, order, rows
 
 def test_more_instances_than_teams_equal_the_oracle():
     syn, B, G = _group(24, 12, 23, 1, 60)
+    (plan,) = cg.solve_plan([G], grid_ctas=20)
+    assert plan["on_chip"] and plan["teams"] < 23
     ((x, xf, dg),) = cg.solve_groups([G], sum_order="rowblock", grid_ctas=20)[0]
     recs = cg.diag_records(dg)
     for m in (0, 11, 22):
@@ -68,6 +72,7 @@ def test_true_residual_in_every_iteration(nrhs):
     streaming kernel (one CTA)."""
     _, _, G = _group(48, 16, 2, nrhs, 25)
     kw = dict(precision="mixed", replace_every=1, replace_above=0.0)
+    assert [cg.solve_plan([G], precision="mixed", grid_ctas=c)[0]["on_chip"] for c in (1, 9, 40, 148)] == [False] + [True] * 3
     (ref,) = cg.solve_groups([G], grid_ctas=1, **kw)
     assert all(r["replacements"] == r["numIters"] > 0 for _, _, d in ref for r in cg.diag_records(d))
     for limit in (9, 40, 148):
