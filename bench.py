@@ -4,7 +4,7 @@
 Workload (one step): a batch of 64 LLC90 instances (13 tiles of 90x90, seeded synthetic ensemble members with
 per-member depth, operator, cg2dNorm and right-hand side), each solved forward (A x = b) and adjoint (A lam = w,
 seeded cotangent w) to a normalised residual of 1e-12 (max 300 iterations each), both right-hand sides of an
-instance sharing its operator in ONE persistent mixed-precision launch, followed by the edge-product kernel
+instance sharing its operator in one mixed-precision call, followed by the edge-product kernel
 (coefficient gradients of J = <w, x>). Unit: forward+adjoint solve pairs per second, whole job.
 
   python bench.py [--gpus N --steps K --warmup W] [--impl reference]
@@ -16,7 +16,7 @@ adjoint solve + coefficient cotangents) on all host cores, one instance per proc
 --mode pressure times SOLVE_FOR_PRESSURE around the solve (update_cg2d, cg2d_rhs, the FP64 solve, the post-solve
 exchange; default batch 16, 50 levels), each step with its own device time and bandwidth.
 
---mode mixed_sizes times one mixed-precision launch over 8 LLC270 and 32 LLC90 instances and reports every
+--mode mixed_sizes times one mixed-precision call over 8 LLC270 and 32 LLC90 instances and reports every
 solution's error against the FP64 solve of the same instance.
 
 --mode exact times the exact-mode adjoint instead (cg2d_adjoint_exact: FP64 forward, then reverse mode through
@@ -247,6 +247,37 @@ def shared_coefficient_bytes(diag_f, diag_a, precision):
     return sum(N_LLC90 * coef * min(f["numIters"], a["numIters"]) for f, a in zip(diag_f, diag_a))
 
 
+def on_chip_bytes(iters, n, precision):
+    """Shared-memory bytes of solves whose state stays on chip: per point-iteration of a right-hand side 15 words (the
+    updates of s and r: 2 read, 1 written each; the stencils A s and M r: 3 read while a warp marches down its rows, 1
+    written each; the x update: 1 read), 60 B in mixed precision, 120 B in FP64."""
+    return sum(iters) * n * 15 * (4 if precision == "mixed" else 8)
+
+
+def solver_launches(plan):
+    """Kernels of one solve call: on chip its launches; streamed one per group for the packed coefficients and the solver."""
+    return max(p["launch"] for p in plan) + 1 if plan[0]["on_chip"] else len(plan) + 1
+
+
+def solver_roofline(plan, streamed, on_chip, ms, sms, sm_mhz, traffic):
+    """The roofline of a solve call. Streamed solves are held against the measured HBM bandwidth. Solves on chip barely touch
+    HBM: they are held against the shared memory's 128 B per clock and SM (at the sampled clock), and the bytes that a
+    streaming kernel would move are given beside it as streamed_model."""
+    peak, kind = measured_peak()
+    gbs = lambda nbytes: nbytes / (ms / 1e3) / 1e9          # noqa: E731
+    if not plan[0]["on_chip"]:
+        return {"bound": "hbm", "achieved": gbs(streamed), "peak": peak, "unit": "GB/s", "frac": gbs(streamed) / peak,
+                "traffic": traffic, "peak_kind": kind, "kernel": "cg2d_persistent (with the FP32 pack)",
+                "kernel_ms": ms, "algorithmic_bytes_per_launch": streamed}
+    smem = 128e-3 * sms * sm_mhz
+    return {"bound": "shared memory", "achieved": gbs(on_chip), "peak": smem, "unit": "GB/s", "frac": gbs(on_chip) / smem,
+            "traffic": traffic, "peak_kind": f"nominal: 128 B per clock, {sms} SMs, {sm_mhz:.0f} MHz",
+            "kernel": "cg2d_team" if len({p["launch"] for p in plan}) == len(plan) else "cg2d_team_groups", "kernel_ms": ms,
+            "algorithmic_bytes_per_launch": on_chip,
+            "streamed_model": {"bytes": streamed, "gbs": gbs(streamed), "of_hbm": gbs(streamed) / peak,
+                               "note": "HBM bytes of a kernel that streams its state; the kernel on chip does not move them"}}
+
+
 def error_vs_fp64(cg, G, slots, L, a):
     """Every member's error against FP64: the same group solved once more in FP64 (ROWBLOCK order, which the tests
     tie to the reference's own solution), outside the timed region; per right-hand side the relative max-norm error
@@ -355,18 +386,26 @@ def run_gpu(a):
     err_fp64 = error_vs_fp64(cg, G, slots, syn.L, a) if a.precision == "mixed" else None
     alg = algorithmic_bytes(diag_f, diag_a, a.precision)
     shared = shared_coefficient_bytes(diag_f, diag_a, a.precision)
-    peak, peak_kind = measured_peak()
     solver_mean = statistics.mean(solver_ms)
-    achieved = alg / (solver_mean / 1e3) / 1e9
+    plan = cg.solve_plan([G], precision=a.precision, **(sched or {}))
     traffic = None
     prof = ROOT / "profiles" / "solver_traffic.json"
     if prof.exists():
-        try:
+        try:   # DRAM bytes of a captured launch of the same kernel, scaled from its instances to this batch
             pj = json.loads(prof.read_text())
-            if pj.get("workload") == f"batch{a.batch}_{a.precision}":
-                traffic = pj.get("bytes_per_launch")
+            if pj.get("kernel") == ("cg2d_team" if plan[0]["on_chip"] else "cg2d_persistent") and \
+                    pj.get("precision") == a.precision:
+                traffic = round(pj["bytes_per_launch"] * a.batch / pj["instances"])
         except Exception:
             traffic = None
+    iters_all = [d["numIters"] for d in diag_f + diag_a]
+    roofline = solver_roofline(plan, alg, on_chip_bytes(iters_all, N_LLC90, a.precision), solver_mean,
+                               torch.cuda.get_device_properties(dev).multi_processor_count,
+                               clocks["sm_mhz"] or clocks["sm_max_mhz"] or 1965.0, traffic)
+    peak = measured_peak()[0]
+    roofline["coefficients_counted_once"] = {
+        "streamed_bytes": alg - shared, "of_hbm": (alg - shared) / (solver_mean / 1e3) / 1e9 / peak,
+        "note": "the 12-word model per solve charges an instance's coefficients to both of its solves"}
 
     # ---- the kernel's own phase timers: one more launch, outside the timed region
     phases = None
@@ -491,18 +530,10 @@ def run_gpu(a):
             "ms_per_step": ms_per_step, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
             "dtype": "f32+f64" if a.precision == "mixed" else "f64", "data": "synthetic",
             "config": arm_config(a, world),
-            "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                         "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind,
-                         "kernel": "cg2d_team (the solver launch)",
-                         "kernel_ms": solver_mean, "algorithmic_bytes_per_launch": alg,
-                         "coefficients_counted_once": {
-                             "algorithmic_bytes_per_launch": alg - shared,
-                             "frac": (alg - shared) / (solver_mean / 1e3) / 1e9 / peak,
-                             "note": "the 12-word model per solve charges an instance's coefficients to both of its "
-                                     "solves; the paired launch reads them once"}},
+            "roofline": roofline,
             "cpu_baseline": cpu,
             "e2e": e2e,
-            "gpu_launches": 2 * a.steps,   # the solve (one team launch) and the edge products
+            "gpu_launches": (solver_launches(plan) + 1) * a.steps,   # the solve and the edge products
             "clocks": clocks,
             "iterations": {"fwd_mean": statistics.mean(d["numIters"] for d in diag_f),
                            "adj_mean": statistics.mean(d["numIters"] for d in diag_a),
@@ -551,15 +582,15 @@ def exact_algorithmic_bytes(iters, checkpoint):
     return tot
 
 
-def exact_launches(kmax, checkpoint):
+def exact_launches(kmax, checkpoint, solver=1):
     """Kernels one cg2d_solve_exact call launches for a batch whose largest iteration count is kmax (memsets
-    excluded): the solve; set-up, neighbour table, r_0 and the scalars from the solve's
+    excluded): the solve (`solver` kernels); set-up, neighbour table, r_0 and the scalars from the solve's
     sums; the cotangent scaling; per iteration two recompute kernels (k_fa, k_fb) and four reverse kernels
     (k_rev_alpha, k_rq, k_rev_beta, k_rz); per segment the alphabar row dots and the two edge-product launches; and
     the two closing kernels."""
     C = checkpoint if checkpoint > 0 else max(1, kmax)
     nseg = -(-kmax // C) if kmax else 0
-    return 1 + 4 + 1 + 6 * kmax + 3 * nseg + 2
+    return solver + 4 + 1 + 6 * kmax + 3 * nseg + 2
 
 
 def _cpu_exact(B, syn, member, iters):
@@ -691,7 +722,8 @@ def run_exact(a):
                      "kernel_ms": ms, "algorithmic_bytes_per_launch": alg},
         "cpu_baseline": cpu,
         "e2e": e2e,
-        "gpu_launches": a.steps * exact_launches(max(iters), a.checkpoint),
+        "gpu_launches": a.steps * exact_launches(max(iters), a.checkpoint, solver_launches(cg.solve_plan(
+            [cg.GroupSpec(ex, ops, [b], [x0], [a.tol], [a.maxit], norms)]))),
         "clocks": clocks,
         "memory": {"peak_allocated_bytes": int(peak_alloc), "resident_inputs_bytes": int(resident),
                    "workspace_bytes": int(ws_bytes)},
@@ -842,7 +874,8 @@ def run_pressure(a):
         "steps_gbs": {"update_cg2d": gbs(upd_b, upd_ms), "cg2d_rhs": gbs(rhs_b, rhs_ms),
                       "cg2d_solve": gbs(solve_alg, solve_ms), "post": gbs(post_b, post_ms)},
         "cpu_baseline": cpu, "e2e": None,
-        "gpu_launches": a.steps * 5,
+        "gpu_launches": a.steps * (4 + solver_launches(cg.solve_plan(
+            [cg.GroupSpec(ex, prev, [st["etaN"]], [st["etaN"]], [a.tol], [a.maxit], norms)]))),
         "clocks": clocks,
         "iterations": {"mean": statistics.mean(r["numIters"] for r in recs), "not_ok":
                        sum(r["status"] != "ok" for r in recs)},
@@ -852,9 +885,9 @@ def run_pressure(a):
 
 
 # ------------------------------------------------------------------------------------------------------------------
-# mixed sizes: LLC270 and LLC90 instances in one mixed-precision launch
+# mixed sizes: LLC270 and LLC90 instances in one mixed-precision call
 
-MIXED_SIZES_METRIC = "CG2D mixed-precision solves/s, 8 LLC270 + 32 LLC90 instances in one launch, on B200"
+MIXED_SIZES_METRIC = "CG2D mixed-precision solves/s, 8 LLC270 + 32 LLC90 instances in one call, on B200"
 
 
 def run_mixed_sizes(a):
@@ -913,21 +946,22 @@ def run_mixed_sizes(a):
                             "mixed_max": max(r["numIters"] for r in recs)}
         bad += sum(r["status"] != "ok" for r in recs)
         alg += sum(n * (r["numIters"] * 56 + r["replacements"] * 96) for r in recs)
-    peak, peak_kind = measured_peak()
-    achieved = alg / (ms / 1e3) / 1e9
+    plan = cg.solve_plan(groups, precision="mixed", **sched)
+    smem_bytes = sum(on_chip_bytes([r["numIters"] for r in cg.diag_records(r_m[0][2])], n, "mixed")
+                     for r_m, n in zip(res, npts))
+    roofline = solver_roofline(plan, alg, smem_bytes, ms, torch.cuda.get_device_properties(dev).multi_processor_count,
+                               clocks["sm_mhz"] or clocks["sm_max_mhz"] or 1965.0, None)
     line = {
         "metric": MIXED_SIZES_METRIC, "value": nsolve / (ms / 1e3), "unit": "solves/s", "n_gpus": 1,
         "steps": a.steps, "warmup": max(3, a.warmup), "ms_per_step": ms, "higher_is_better": True,
         "scaling": "weak", "vs_baseline": None, "dtype": "f32+f64", "data": "synthetic",
-        "config": {"workload": "8 LLC270 + 32 LLC90 instances (two groups) in one mixed-precision persistent launch, "
+        "config": {"workload": "8 LLC270 + 32 LLC90 instances (two groups) in one mixed-precision call, "
                                f"to {a.tol:g} (LLC270 cap 1000 iterations, LLC90 {a.maxit})",
                    "grid": "LLC270 13x270x270 and LLC90 13x90x90, halo 4", "l2": "inputs larger than L2 (no flush)",
                    "parallelism": "1 GPU"},
-        "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                     "traffic": None, "peak_kind": peak_kind, "kernel": "cg2d_team (mixed, one launch per group)",
-                     "kernel_ms": ms, "algorithmic_bytes_per_launch": alg},
+        "roofline": roofline,
         "error_vs_f64": errs, "iterations": iters, "not_ok": bad,
-        "cpu_baseline": None, "e2e": None, "gpu_launches": 2 * a.steps, "clocks": clocks,
+        "cpu_baseline": None, "e2e": None, "gpu_launches": solver_launches(plan) * a.steps, "clocks": clocks,
         "schedule": {"chosen": sched, "launch": "CUDA graph replay"},
     }
     print(json.dumps(line))

@@ -27,3 +27,24 @@ def test_shared_coefficients_counted_while_both_solves_iterate():
     both = bench.algorithmic_bytes([_d(100)], [_d(100)], "mixed") - bench.shared_coefficient_bytes(
         [_d(100)], [_d(100)], "mixed")
     assert both == n * 100 * 88
+
+
+def _plan(*launches, on_chip=True):
+    return [{"launch": n, "on_chip": on_chip, "teams": 1, "ctas_per_team": 1} for n in launches]
+
+
+def test_roofline_and_launches_follow_the_route():
+    """A solve on chip is held against the shared memory (60 B a point-iteration of a right-hand side in mixed precision, 120
+    B in FP64) with the streaming kernel's bytes beside it; a streamed one against HBM. The launch counts are the plan's."""
+    n = bench.N_LLC90
+    assert bench.on_chip_bytes([240, 230], n, "mixed") == n * 470 * 60
+    assert bench.on_chip_bytes([1], 10, "f64") == 1200
+    r = bench.solver_roofline(_plan(0), 4e9, 2e9, 1.0, 148, 1965.0, None)
+    assert r["bound"] == "shared memory" and r["kernel"] == "cg2d_team" and r["achieved"] == 2000.0
+    assert abs(r["peak"] - 148 * 128 * 1.965) < 1e-6 and r["streamed_model"]["bytes"] == 4e9
+    assert bench.solver_roofline(_plan(0, 0), 4e9, 2e9, 1.0, 148, 1965.0, None)["kernel"] == "cg2d_team_groups"
+    r = bench.solver_roofline(_plan(0, 0, on_chip=False), 4e9, 2e9, 1.0, 148, 1965.0, 5)
+    assert r["bound"] == "hbm" and r["achieved"] == 4000.0 and r["traffic"] == 5 and r["peak"] == bench.measured_peak()[0]
+    assert [bench.solver_launches(p) for p in (_plan(0), _plan(0, 0, 1), _plan(0, on_chip=False),
+                                               _plan(0, 0, on_chip=False))] == [1, 2, 2, 3]
+    assert bench.exact_launches(30, 30, 2) == bench.exact_launches(30, 30) + 1
