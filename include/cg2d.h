@@ -14,7 +14,7 @@
  *                          the exch2 halo map becomes per-tile-edge neighbour tables read by the stencil.
  *   cg2d_solve_f64         cg2d_fortran(ex, ops, cg2d_b, cg2d_x, ...) (mitgcm_jax/core/cg2d.py:205-269),
  *                          batched; cg2d_solve (cg2d.py:351-375) is this call plus the Python-side mask.
- *   cg2d_solve_groups      the same solver for several uniform batches in one persistent launch
+ *   cg2d_solve_groups      the same solver for several uniform batches in one call
  *                          (mixed LLC90/LLC270 batches, forward + adjoint right-hand sides sharing
  *                          one operator).
  *   cg2d_apply_operator    _matvec (cg2d.py:292-298): (A / cg2dNorm) v on the interior, 0 on halos.
@@ -55,7 +55,7 @@ typedef enum {
      order from 0 (global_sum.py:20-26). Same result for every launch geometry. */
   CG2D_SUM_ROWBLOCK = 0,
   /* "fortran" order of cg2d.py:141-161: s = 0; DO j; DO i; s = s + a(i,j), then the tiles in
-     order from 0. Bitwise equal to the reference's sum_order="fortran"; slow (one thread per tile). */
+     order from 0. Bitwise equal to the reference's sum_order="fortran"; slow (a tile's additions are one chain). */
   CG2D_SUM_FORTRAN = 1
 } cg2d_sum_order_t;
 
@@ -74,9 +74,10 @@ typedef struct {
   int ctas_per_sm;     /* 0 = occupancy maximum. FP64 has two kernel builds: for 1 CTA per SM and for 2 (fewer
                           registers a thread). 2 takes the second; 0 takes it when every group has one right-hand
                           side and there are at least 8 work units per SM, otherwise the first. Results-neutral */
-  double timeout_s;    /* bound on every grid-wide wait (default 10 s) */
+  double timeout_s;    /* bound on every wait of a kernel (default 10 s) */
   int test_missing_arrivals; /* testing only (default 0): the first grid-wide wait expects this many
-                                arrivals more than there are CTAs, so it runs out after timeout_s and
+                                arrivals more than there are CTAs (on chip: the first wait is for a message
+                                that nobody sends), so it runs out after timeout_s and
                                 every solve reports CG2D_BARRIER_TIMEOUT (exercises the bounded wait) */
   int profile;         /* 1: record per-CTA phase times in the workspace (cg2d_workspace_profile) */
   int unit_deal;       /* how the work units (instance, tile, row block) are dealt to the CTAs:
@@ -144,7 +145,8 @@ typedef struct {
 
 void cg2d_default_params(cg2d_params_t* p);
 
-/* Bytes of device workspace for a cg2d_solve_groups call with these groups. */
+/* Bytes of device workspace for a cg2d_solve_groups call with these groups, on chip or streamed (solves on chip use a part
+ * of it). */
 size_t cg2d_workspace_size(const cg2d_group_t* groups, int ngroups, const cg2d_params_t* params);
 
 /* How a cg2d_solve_groups call with these groups and parameters would run (sizes and parameters decide; nothing is

@@ -17,14 +17,16 @@
 // sends the halo values h + 2 only after an exchange that every reader of h has entered having read h.
 //
 // Teams never wait for one another. An instance is as large as its team's shared memory (team_plan); what does not
-// fit runs in cg2d_solver.cu, which streams the state. The arithmetic, the sum order and the results are those of
+// fit runs in cg2d_solver.cu, which streams the state. Groups of a call have a launch each (cg2d_team) or share one on parts
+// of the CTAs (cg2d_team_groups). The arithmetic, the sum order and the results are those of
 // cg2d_solver.cu bit for bit, in every precision and sum order.
 //
 // What bounds it. One LLC90 FP64 solve: 2.3 ms, 4.6 us a pass (6.9 ms and 14 us when streamed): the message latency (an
 // all-to-all of 148 CTAs takes 1.3 us when every CTA's sums have 128-byte lines of their own, 3.2 us when CTAs share
 // lines), the block barriers and short dependent steps between the phases. Batches: the shared-memory / L1 pipe. With 11
-// teams of 13 CTAs (mixed pairs) it is busy 54 % of the time, DRAM 2 %, issue slots 37 %; 64 mixed pairs take 31 ms (48
-// streamed), 64 FP64 solves 29 ms (52). One LLC270 FP64 solve: 16 ms (54).
+// teams of 13 CTAs (mixed pairs) it is busy 53 % of the time, DRAM 2 %, issue slots 37 %; 64 mixed pairs take 31 ms (48
+// streamed), 64 FP64 solves 29 ms (52). One LLC270 FP64 solve: 16 ms (54); nothing is near its peak (shared-memory / L1 pipe
+// 46 %, issue slots 32 %, DRAM 2 %), warps wait at block barriers (24 rows over 16 warps) and for shared memory.
 // Two CTAs of 8 warps per SM, so that one team computes while another waits, measured the same (16 FP64 solves 8.7 ms
 // either way) and fit fewer teams.
 
@@ -528,7 +530,8 @@ struct Team {
   }
   // the sum of the products a b of nj rows of n points in order, rows ap and bp elements apart, by one warp: the lanes form
   // 32 consecutive products and every lane adds them in order from
-  // shuffles, which do not depend on the additions, so that the chain runs near the latency of one addition (8.7 cycles).
+  // shuffles, which do not depend on the additions. 14 cycles a product with two chains on an SM (a dependent addition takes
+  // 8.7; the rest, not shown by measurement, likely goes to the products' loads and addresses between the blocks of 32).
   // A function of its own: inlined into the pass, the compiler issues each shuffle only behind the addition before it, for
   // want of registers (32 cycles a product). Zeros past the end leave the sum as it is (it starts at +0, so it never is -0).
   __device__ __noinline__ static double chain(const T* a, const T* b, int bp, int s, int n, int nj, int ap) {
@@ -1382,7 +1385,8 @@ size_t smem_layout(const TopoDev& tp, int nrhs, int mixed, int rows, int ring, i
 }
 
 // Time of a pass in units of an exchange (4.2 us with its fixed steps): 1 + kRowCost per row of the largest CTA's warps and
-// 32 columns. Measured, LLC90 FP64: 4.6 us at 8 rows a CTA, 9.1 us at 66, 10.6 us at 90. In the FORTRAN order also a tile's
+// 32 columns, whatever the precision, the right-hand sides and the number of messages (only splits of one launch are
+// compared). Fitted to LLC90 FP64: 4.6 us at 8 rows a CTA, 9.1 us at 66, 10.6 us at 90. In the FORTRAN order also a tile's
 // additions: a CTA's n ordered sums run side by side on its warps, at 11.5 + 1.05 n cycles an addition (latency and
 // shuffles). Measured: 14 cycles with 2 sums, 15 with 4, 19 with 8, 26 with 12 and 14: LLC90 73 us a pass with 1 tile a CTA,
 // 82 us with 2; LLC32 9.6 us with 1, 23 us with 7.

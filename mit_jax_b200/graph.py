@@ -2,8 +2,8 @@
 
 `GraphedSolve` records one `solve_groups` call, and optionally work that follows it on the same stream (the edge
 products of an adjoint, say), into a torch.cuda.CUDAGraph. A replay re-runs the whole sequence: the workspace
-clear, the coefficient packing, the persistent cooperative kernel and the follow-up kernels, with no Python and
-no per-launch host work. The groups' tensors are the graph's static inputs: write new values into them in place
+clear, the solver's persistent kernels (and the coefficient packing where it streams) and the follow-up kernels, with
+no Python and no per-launch host work. The groups' tensors are the graph's static inputs: write new values into them in place
 (`copy_`) between replays. The outputs are static too: replay() returns the same tensors every time, overwritten.
 
 Capture rules the class takes care of:
