@@ -149,8 +149,8 @@ void cg2d_default_params(cg2d_params_t* p);
  * of it). */
 size_t cg2d_workspace_size(const cg2d_group_t* groups, int ngroups, const cg2d_params_t* params);
 
-/* How a cg2d_solve_groups call with these groups and parameters would run (sizes and parameters decide; nothing is
- * launched). One entry per group. */
+/* How a cg2d_solve_groups call with these groups and parameters, and a workspace of cg2d_workspace_size, would run (sizes
+ * and parameters decide; nothing is launched). One entry per group. */
 typedef struct {
   int on_chip;         /* 1: an instance's state stays in the shared memory of a team of CTAs; 0: it is streamed */
   int launch;          /* the solver launch that runs the group: 0 .. launches - 1; groups may share one */

@@ -94,3 +94,14 @@ def test_struct_layouts_match_the_c_compiler(tmp_path):
         assert int(got[cname]) == ctypes.sizeof(st), cname
         for f, _ in st._fields_:
             assert int(got[f"{cname}.{f}"]) == getattr(st, f).offset, (cname, f)
+
+
+def test_plan_struct_and_bad_arguments_without_a_gpu():
+    lib = capi.lib()
+    assert ctypes.sizeof(capi.GroupPlan) == 16
+    g, plan = (capi.Group * 1)(), (capi.GroupPlan * 1)()
+    assert lib.cg2d_plan(g, 1, None, plan) == capi.CG2D_BAD_ARG            # no topology
+    assert lib.cg2d_plan(g, 1, None, None) == capi.CG2D_BAD_ARG
+    p = capi.default_params()
+    p.rows_per_block = 7
+    assert lib.cg2d_plan(g, 1, ctypes.byref(p), plan) == capi.CG2D_BAD_ARG
