@@ -202,7 +202,7 @@ void team_layout(const cg2d_group_t* gr, int ng, const cg2d_params_t* p, WsLayou
       const TopoDev tp = topo_dev(gr[g].topo);
       least[g] = team_least_ctas(tp, gr[g].nrhs, mixed, serial, L->t[g]);
       if (least[g] == 0 || least[g] > ctas) { fits = false; break; }
-      est[g] = team_cost(tp, gr[g].count, gr[g].nrhs, serial, least[g], ctas, L->t[g]);
+      est[g] = team_cost(tp, gr[g].count, gr[g].nrhs, mixed, serial, least[g], ctas, L->t[g]);
     }
     if (fits) {
       double cost[kMaxGroups + 1];   // of groups 0 .. b - 1
@@ -216,7 +216,7 @@ void team_layout(const cg2d_group_t* gr, int ng, const cg2d_params_t* p, WsLayou
           double slowest = 0.0, sum = 0.0;
           bool ok = true;
           for (int g = a; g < b && ok; ++g) {
-            const double c = team_cost(topo_dev(gr[g].topo), gr[g].count, gr[g].nrhs, serial, least[g], part[g], L->t[g]);
+            const double c = team_cost(topo_dev(gr[g].topo), gr[g].count, gr[g].nrhs, mixed, serial, least[g], part[g], L->t[g]);
             ok = c <= kShareSlow * est[g];
             slowest = c > slowest ? c : slowest;
             sum += est[g];

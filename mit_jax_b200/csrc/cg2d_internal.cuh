@@ -272,7 +272,7 @@ cudaError_t solver_occupancy(const KParams& kp, size_t smem, int* blocks_per_sm)
 size_t team_plan(const TopoDev& tp, int count, int nrhs, int mixed, int serial, int ctas, TeamDev* t, double* cost);
 // The same without the split itself: CTAs of a team that surely fits (0: none), and the cost on `ctas` CTAs at that size or above
 int team_least_ctas(const TopoDev& tp, int nrhs, int mixed, int serial, const TeamDev& t);
-double team_cost(const TopoDev& tp, int count, int nrhs, int serial, int least, int ctas, const TeamDev& t);
+double team_cost(const TopoDev& tp, int count, int nrhs, int mixed, int serial, int least, int ctas, const TeamDev& t);
 size_t team_msg_bytes(const TopoDev& tp, int nrhs, int mixed, const TeamDev& t);   // per team
 size_t team_coef_bytes(const TopoDev& tp, int mixed, const TeamDev& t);            // per team
 cudaError_t launch_team(const TeamParams& kp, int mixed, int serial, size_t smem, cudaStream_t stream);

@@ -1384,20 +1384,29 @@ size_t smem_layout(const TopoDev& tp, int nrhs, int mixed, int rows, int ring, i
   return o;
 }
 
-// Time of a pass in units of an exchange (4.2 us with its fixed steps): 1 + kRowCost per row of the largest CTA's warps and
-// 32 columns, whatever the precision, the right-hand sides and the number of messages (only splits of one launch are
-// compared). Fitted to LLC90 FP64: 4.6 us at 8 rows a CTA, 9.1 us at 66, 10.6 us at 90. In the FORTRAN order also a tile's
-// additions: a CTA's n ordered sums run side by side on its warps, at 11.5 + 1.05 n cycles an addition (latency and
-// shuffles). Measured: 14 cycles with 2 sums, 15 with 4, 19 with 8, 26 with 12 and 14: LLC90 73 us a pass with 1 tile a CTA,
-// 82 us with 2; LLC32 9.6 us with 1, 23 us with 7.
-double pass_cost(const TopoDev& tp, int nrhs, int serial, int rows, int units) {
-  const double kRowCost = 0.09, kExchangeCycles = 8064.0, steps = (tp.ni + 31) / 32;
-  double pass = 1.0 + kRowCost * ((rows + kTeamWarps - 1) / kTeamWarps) * steps;
-  if (serial) {
-    const int sums = 2 * nrhs * units, turns = (sums + kTeamWarps - 1) / kTeamWarps;
-    pass += (double)tp.ni * tp.nj * (11.5 * turns + 1.05 * sums) / kExchangeCycles;
-  }
-  return pass;
+// Time of a pass in units of an exchange (4.2 us with its fixed steps); only splits of one launch and the groups of one call
+// are compared. From rows alone: 1 + kRowCost per row of the largest CTA's warps and 32 columns, whatever the precision and
+// the right-hand sides. Fitted to LLC90 FP64: 4.6 us at 8 rows a CTA, 9.1 us at 66, 10.6 us at 90.
+double row_cost(const TopoDev& tp, int rows) {
+  const double kRowCost = 0.09;
+  return 1.0 + kRowCost * ((rows + kTeamWarps - 1) / kTeamWarps) * ((tp.ni + 31) / 32);
+}
+// In the FORTRAN order with the ordered additions, too. A CTA's n sums (two kinds in pass X, one in pass S) run side by side on
+// its warps, at 15.6 cycles an addition until their shuffles fill the SM at 2.28 cycles an addition and sum. Fitted to 288
+// workloads of 2 to 128 instances with tiles of 8 to 96 points, in two splits each, to 2.3 % (root mean square).
+double pass_cost(const TopoDev& tp, int nrhs, int mixed, int serial, int rows, int units) {
+  if (!serial) return row_cost(tp, rows);
+  const double steps = (tp.ni + 31) / 32, per_warp = (rows + kTeamWarps - 1) / kTeamWarps;
+  auto chains = [&](int n) {   // cycles an addition of n sums takes
+    const int rem = n % kTeamWarps;
+    double c = n / kTeamWarps * 2.28 * kTeamWarps;
+    if (rem) c += 2.28 * rem > 15.6 ? 2.28 * rem : 15.6;
+    return c;
+  };
+  const double row = mixed ? (nrhs == 2 ? 0.34 : 0.28) : (nrhs == 2 ? 0.57 : 0.33);
+  const double us = 3.3 + 0.0096 * nrhs * tp.T + per_warp * (0.44 + row * steps) +
+                    (double)tp.ni * tp.nj * (chains(2 * nrhs * units) + chains(nrhs * units)) / 2 / 1920.0;
+  return us / 4.2;
 }
 
 }  // namespace
@@ -1408,9 +1417,14 @@ size_t team_plan(const TopoDev& tp, int count, int nrhs, int mixed, int serial, 
   const int nj = tp.nj, ni = tp.ni, rows = tp.T * nj;
   t->nslots = (2ll * rows + 2ll * t->units * ni + 7) & ~7ll;   // (whole 128-byte lines)
   if (t->nslots > (1ll << 30)) return 0;
-  // The split with the least rounds x pass time is taken: 16 ROWBLOCK solves run 8 teams of 18 CTAs, 64 run 11 teams of 13;
-  // 64 mixed LLC90 solves in the FORTRAN order run 21 teams of 7 in 4 rounds (14.0 ms for 20 iterations), not 11 teams of 13
-  // in 6 (19.0 ms; 16.3 streamed).
+  // The split with the least rounds x pass time is taken: 16 ROWBLOCK solves run 8 teams of 18 CTAs, 64 run 11 teams of 13.
+  // FORTRAN order: the split that is the best by rows, unless the estimate with the ordered additions has another one at
+  // least kSure faster (it is good to 2 or 3 %). 64 mixed LLC90 solves run 21 teams of 7 in 4 rounds (14.0 ms for 20
+  // iterations), not the 11 teams of 13 in 6 that the rows alone give (19.0 ms; 16.3 streamed).
+  const double kSure = 0.96;
+  double rows_best = 0.0, rows_pass = 0.0;
+  size_t rows_smem = 0;
+  TeamDev by_rows;
   double best = 0.0;
   size_t best_smem = 0;
   TeamDev cand = *t;
@@ -1449,12 +1463,24 @@ size_t team_plan(const TopoDev& tp, int count, int nrhs, int mixed, int serial, 
     const size_t o = smem_layout(tp, nrhs, mixed, max_rows, max_ring, max_halo, max_units, &cand);
     if (o > (size_t)kSmemLimit) continue;
     const int rounds = (count + cand.nteams - 1) / cand.nteams;
-    const double c = rounds * pass_cost(tp, nrhs, serial, max_rows, max_units);
+    const double c = rounds * pass_cost(tp, nrhs, mixed, serial, max_rows, max_units);
     if (best_smem == 0 || c < best) {
       best = c;
       best_smem = o;
       *t = cand;
     }
+    const double r = rounds * row_cost(tp, max_rows);
+    if (rows_smem == 0 || r < rows_best) {
+      rows_best = r;
+      rows_pass = c;
+      rows_smem = o;
+      by_rows = cand;
+    }
+  }
+  if (rows_smem != 0 && best > kSure * rows_pass) {
+    best = rows_pass;
+    best_smem = rows_smem;
+    *t = by_rows;
   }
   *cost = best;
   return best_smem;
@@ -1479,7 +1505,7 @@ int team_least_ctas(const TopoDev& tp, int nrhs, int mixed, int serial, const Te
   return (t.units + lo - 1) / lo;
 }
 
-double team_cost(const TopoDev& tp, int count, int nrhs, int serial, int least, int ctas, const TeamDev& t) {
+double team_cost(const TopoDev& tp, int count, int nrhs, int mixed, int serial, int least, int ctas, const TeamDev& t) {
   if (ctas > kTeamMaxCtas) ctas = kTeamMaxCtas;
   double best = 0.0;
   for (int nt = 1; nt <= count && nt * least <= ctas; ++nt) {
@@ -1487,7 +1513,7 @@ double team_cost(const TopoDev& tp, int count, int nrhs, int serial, int least, 
     const int units = (t.units + G - 1) / G, nteams = ctas / G < count ? ctas / G : count;
     int rows = (tp.T * tp.nj + G - 1) / G + (G < t.units ? t.rpb / 2 : 0);   // (runs end at units)
     if (serial || rows > units * t.rpb) rows = units * t.rpb;
-    const double c = (count + nteams - 1) / nteams * pass_cost(tp, nrhs, serial, rows, units);
+    const double c = (count + nteams - 1) / nteams * pass_cost(tp, nrhs, mixed, serial, rows, units);
     if (best == 0.0 || c < best) best = c;
   }
   return best;
