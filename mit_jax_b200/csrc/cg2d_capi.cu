@@ -152,28 +152,41 @@ cg2d_status_t size_stages(const cg2d_group_t* gr, int ng, int mixed, int serial,
 // pass takes more than kShareSlow times as long as alone and the slowest pass at most kShareGain of the passes one after the
 // other. Measured (us for 40 iterations of every group: streamed, one after the other, shared): 4 x LLC8 973, 1250, 409; 2 and
 // 4 x LLC90 FP64 1545, 882, 563 and 2114, 1722, 762; 4 x LLC90 FORTRAN order 9756, 23307, 6257; LLC8 + 16 + 32 + 90 1402,
-// 1392, 518. (With different iteration counts the longest group decides: alone among ended ones, one of 4 x LLC90 takes 8.7 us
-// a pass on its quarter of the chip, 4.6 on all of it, 14 streamed.) Not shared, for want of CTAs: 2 x 16 LLC90 FP64 5665,
-// 3426, -; 2 LLC270 + 8 LLC90 mixed pairs (20 iterations) 5946, 1892, -.
-constexpr double kShareSlow = 1.5, kShareGain = 0.8;
+// 1392, 540. Not shared, for want of CTAs: 2 x 16 LLC90 FP64 5665, 3426, -; 2 LLC270 + 8 LLC90 mixed pairs (20 iterations)
+// 5946, 1892, -. Of 280 random sets of 2 to 4 groups none was slower than streamed (0.35 to 0.84 of its time); with the same
+// iteration count in every group none was slower than one after the other, with counts from 8 to 60 four were, the worst 1.16
+// times (there a group that shares its launch with ended ones runs on).
+constexpr double kShareSlow = 1.45, kShareGain = 0.7;
 
-// the parts of `ctas` CTAs that groups a .. b - 1 get in a shared launch: the least each needs, and the rest by their rows;
-// false when they do not fit side by side
-bool share_ctas(const cg2d_group_t* gr, const WsLayout* L, const int* least, int a, int b, int ctas, int* part) {
-  double work[kMaxGroups], all = 0.0;
-  int left = ctas;
-  for (int g = a; g < b; ++g) {
-    left -= least[g];
-    work[g] = (double)gr[g].count * gr[g].topo->nTiles * gr[g].topo->sNy * ((gr[g].topo->sNx + 31) / 32);
-    all += work[g];
+// The parts of `ctas` CTAs that groups a .. b - 1 get in a shared launch, at least `least` and at most `used` (alone) each;
+// false when they do not fit side by side. All get slower by the same factor f, as nearly as that goes, so that no group is
+// starved whatever the iteration counts: a pass of cost `est` alone takes est - work / used + work / part on a part.
+bool share_ctas(const cg2d_group_t* gr, const int* least, const int* used, const double* est, int a, int b, int ctas,
+                int* part) {
+  int need = 0;
+  for (int g = a; g < b; ++g) need += least[g];
+  if (need > ctas) return false;
+  auto parts = [&](double f) {
+    int all = 0;
+    for (int g = a; g < b; ++g) {
+      const cg2d_topology* tp = gr[g].topo;
+      const double work = 0.09 / kTeamWarps * gr[g].count * tp->nTiles * tp->sNy * ((tp->sNx + 31) / 32);
+      const double p = work / ((f - 1.0) * est[g] + work / used[g]);
+      part[g] = p < used[g] ? (int)std::ceil(p) : used[g];
+      if (part[g] < least[g]) part[g] = least[g];
+      all += part[g];
+    }
+    return all;
+  };
+  if (parts(1.0) <= ctas) return true;
+  double lo = 1.0, hi = 2.0;
+  while (parts(hi) > ctas && hi < 1e6) hi *= 2.0;
+  for (int i = 0; i < 12; ++i) {
+    const double mid = 0.5 * (lo + hi);
+    if (parts(mid) <= ctas) hi = mid;
+    else lo = mid;
   }
-  if (left < 0) return false;
-  for (int g = a; g < b; ++g) {
-    const long long most = (long long)gr[g].count * L->units[g];   // (a CTA has at least one unit)
-    const long long p = least[g] + (long long)(left * work[g] / all);
-    part[g] = (int)(p < most ? p : most);
-  }
-  return true;
+  return parts(hi) <= ctas;
 }
 
 void team_layout(const cg2d_group_t* gr, int ng, const cg2d_params_t* p, WsLayout* L) {
@@ -195,13 +208,15 @@ void team_layout(const cg2d_group_t* gr, int ng, const cg2d_params_t* p, WsLayou
   }
   if (ng > 1) {
     // the cheapest cut of the groups into launches, by estimate
-    int least[kMaxGroups], part[kMaxGroups];
+    int least[kMaxGroups], used[kMaxGroups], part[kMaxGroups];
     double est[kMaxGroups];
     bool fits = true;
     for (int g = 0; g < ng; ++g) {
       const TopoDev tp = topo_dev(gr[g].topo);
       least[g] = team_least_ctas(tp, gr[g].nrhs, mixed, serial, L->t[g]);
-      if (least[g] == 0 || least[g] > ctas) { fits = false; break; }
+      used[g] = L->t[g].G * L->t[g].nteams;
+      if (least[g] > used[g]) least[g] = used[g];   // (the estimate is on the safe side)
+      if (least[g] == 0) { fits = false; break; }
       est[g] = team_cost(tp, gr[g].count, gr[g].nrhs, mixed, serial, least[g], ctas, L->t[g]);
     }
     if (fits) {
@@ -212,7 +227,7 @@ void team_layout(const cg2d_group_t* gr, int ng, const cg2d_params_t* p, WsLayou
         cost[b] = cost[b - 1] + est[b - 1];
         from[b] = b - 1;
         for (int a = b - 2; a >= 0; --a) {
-          if (!share_ctas(gr, L, least, a, b, ctas, part)) break;
+          if (!share_ctas(gr, least, used, est, a, b, ctas, part)) break;
           double slowest = 0.0, sum = 0.0;
           bool ok = true;
           for (int g = a; g < b && ok; ++g) {
@@ -230,7 +245,7 @@ void team_layout(const cg2d_group_t* gr, int ng, const cg2d_params_t* p, WsLayou
       // the splits of the shared launches; one that turns out not to fit or not to pay has its groups one after the other
       for (int b = ng; b > 0; b = from[b]) {
         const int a = from[b];
-        if (b - a < 2 || !share_ctas(gr, L, least, a, b, ctas, part)) continue;
+        if (b - a < 2 || !share_ctas(gr, least, used, est, a, b, ctas, part)) continue;
         TeamDev t[kMaxGroups];
         size_t smem[kMaxGroups];
         double slowest = 0.0, sum = 0.0;

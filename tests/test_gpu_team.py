@@ -164,3 +164,13 @@ def test_split_by_rows_is_overruled_only_when_sure(N, ts, count, nrhs, teams, ct
     to 9 % slower."""
     (plan,) = cg.solve_plan([_sizes_only(N, ts, count, nrhs)], precision="mixed", sum_order="fortran")
     assert (plan["teams"], plan["ctas_per_team"]) == (teams, ctas)
+
+
+def test_no_group_of_a_shared_launch_is_starved():
+    """Each group gets the CTAs that slow it down as much as the others. A group of small tiles beside a large one, which by its
+    rows would get a CTA a team, keeps its 13; and a group that needs a CTA per tile does not keep the others from sharing."""
+    plan = cg.solve_plan([_sizes_only(8, 8, 2, 1), _sizes_only(180, 180, 1, 1)])
+    assert all(p["on_chip"] for p in plan)
+    assert plan[0]["launch"] != plan[1]["launch"] or plan[0]["ctas_per_team"] >= 7, plan
+    plan = cg.solve_plan([_sizes_only(90, 90, 1, 1), _sizes_only(32, 32, 2, 1), _sizes_only(90, 90, 5, 1)], sum_order="fortran")
+    assert [p["launch"] for p in plan] == [0, 0, 0] and [p["ctas_per_team"] for p in plan] == [13, 13, 13], plan
